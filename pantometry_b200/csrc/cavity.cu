@@ -572,7 +572,6 @@ struct Cavity : Handle {
         n.current = t.current; n.ncurrent = t.ncurrent;
         n.eps_src = t.eps_src; n.sig_src = t.sig_src;
         n.dt = h; n.volume = t.volume; n.g = t.g; n.eps_u = t.eps_u; n.mu_u = t.mu_u;
-        n.st = t.st;
         return n;
     }
     // The box's f64 values from the stored field of the present parity.

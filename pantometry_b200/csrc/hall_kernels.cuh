@@ -228,8 +228,7 @@ __device__ __forceinline__ void hall_stage(unsigned base, unsigned halo_at, cons
 // work, the startup offset on the first step (hall.rs:513-528) and the audit.
 template <typename Real>
 __device__ __forceinline__ void hall_finish(const HallArgs<Real>& a, double (&acc)[3], double delta) {
-    DevState* st = a.st;
-    if (finish_blocks<3>(acc, a.partials, a.nblocks, &st->counter) && linear_tid() == 0) {
+    close_books<3>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double plus = acc[0];
         st->injected += acc[2];
         st->last_delta = delta;
@@ -257,7 +256,7 @@ __device__ __forceinline__ void hall_finish(const HallArgs<Real>& a, double (&ac
         st->part[0] = total;
         st->invariant = plus;
         audit_and_commit(st, total, scale);
-    }
+    });
 }
 
 template <typename Real, bool HET>

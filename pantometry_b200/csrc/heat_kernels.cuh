@@ -293,8 +293,7 @@ __device__ __forceinline__ void tile_column(const Tiles& T, long long t, int& i,
 // acc: stored heat, heat shed, and (filled blocks) heat generated.
 template <int NV>
 __device__ __forceinline__ void heat_plain_books(const HeatPlainArgs& a, double (&acc)[NV]) {
-    if (finish_blocks<NV>(acc, a.partials, a.nblocks, &a.st->counter) && linear_tid() == 0) {
-        DevState* st = a.st;
+    close_books<NV>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         st->lost += acc[1];
         if constexpr (NV > 2) st->supplied += acc[2];
         double total = 0.0, scale = 0.0;
@@ -306,10 +305,11 @@ __device__ __forceinline__ void heat_plain_books(const HeatPlainArgs& a, double 
         st->part[2] = -st->supplied;
         audit_and_commit(st, total, scale);
         if (a.radiating) {  // worst_rate_now of the state this step leaves (solid.rs:1148-1185)
-            const unsigned long long bits = atomicExch(&st->rate_bits, 0ull);
+            const unsigned long long bits = st->rate_bits;
+            st->rate_bits = 0ull;
             st->rate_now = bits ? fmax(a.static_rate, __longlong_as_double((long long)bits)) : a.static_rate;
         }
-    }
+    });
 }
 
 // Plain form. Each thread marches its column through the tile's planes, holding the cell
@@ -644,8 +644,7 @@ struct HeatF32Args {
 // acc: stored heat, heat shed, and (filled blocks) heat generated.
 template <int NV>
 __device__ __forceinline__ void heat_f32_books(const HeatF32Args& a, double (&acc)[NV], bool filled) {
-    if (finish_blocks<NV>(acc, a.partials, a.nblocks, &a.st->counter) && linear_tid() == 0) {
-        DevState* st = a.st;
+    close_books<NV>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double stored = filled ? acc[0] : a.capacity * acc[0];
         st->lost += filled ? acc[1] : a.capacity * acc[1];
         if constexpr (NV > 2) st->supplied += acc[2];
@@ -658,10 +657,11 @@ __device__ __forceinline__ void heat_f32_books(const HeatF32Args& a, double (&ac
         st->part[2] = -st->supplied;
         audit_and_commit(st, total, scale);
         if (a.radiating) {  // worst_rate_now of the state this step leaves (solid.rs:1148-1185)
-            const unsigned long long bits = atomicExch(&st->rate_bits, 0ull);
+            const unsigned long long bits = st->rate_bits;
+            st->rate_bits = 0ull;
             st->rate_now = bits ? fmax(a.rad.static_rate, __longlong_as_double((long long)bits)) : a.rad.static_rate;
         }
-    }
+    });
 }
 
 // Chosen form, z-marching like the plain form; neighbours in the plane come from L1/L2.
@@ -953,7 +953,7 @@ static __global__ void __launch_bounds__(256) bar_step(BarArgs<Real> a) {
         a.tnew[i] = nt;
         acc[0] += (double)nt - a.reference;
     }
-    if (finish_blocks<1>(acc, a.partials, a.nblocks, &st->counter) && linear_tid() == 0) {
+    close_books<1>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double stored = a.capacity * acc[0];
         double total = 0.0, scale = 0.0;
         ledger_add(total, scale, stored);
@@ -961,7 +961,7 @@ static __global__ void __launch_bounds__(256) bar_step(BarArgs<Real> a) {
         st->part[0] = stored;
         st->part[1] = st->injected;
         audit_and_commit(st, total, scale);
-    }
+    });
 }
 
 template <typename Real>

@@ -11,7 +11,7 @@
 // mbarrier is bounded; a wait that runs out stops the call with kDeviceTimeout.
 //
 // The books: each thread sums its cells' new deviations and the heat its films shed in FP64; the
-// grid's sums are reduced in fixed order by the last CTA (finish_blocks), which runs the ledger and
+// grid's sums are reduced in fixed order by the last CTA (close_books), which runs the ledger and
 // the audit as heat_f32_step does.
 #pragma once
 
@@ -110,7 +110,7 @@ static __global__ void __launch_bounds__(kEnsConsumers + 32, PM_ENS_TMA_MIN_BLOC
         }
     }
     if (__syncthreads_or(timed_out ? 1 : 0)) return;
-    if (finish_blocks<2>(acc, a.partials, a.nblocks, &st->counter) && tid == 0) {
+    close_books<2>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double stored = a.capacity * acc[0];
         st->lost += a.capacity * acc[1];
         double total = 0.0, scale = 0.0;
@@ -121,7 +121,7 @@ static __global__ void __launch_bounds__(kEnsConsumers + 32, PM_ENS_TMA_MIN_BLOC
         st->part[1] = st->lost;
         st->part[2] = -st->supplied;
         audit_and_commit(st, total, scale);
-    }
+    });
 }
 
 }  // namespace pm

@@ -67,7 +67,7 @@ static __global__ void __launch_bounds__(256) room_step(RoomArgs<Real> a) {
         const double dr = (double)right, da = (double)above;
         acc[0] += (si * sj) * a.knode * (double)np * (double)pc + sj * a.kface * (dr * dr) + si * a.kface * (da * da);
     }
-    if (finish_blocks<1>(acc, a.partials, a.nblocks, &st->counter) && linear_tid() == 0) {
+    close_books<1>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double invariant = acc[0];
         if (a.starting) {
             // room.rs:448-476: the released state's datum against the staggered invariant
@@ -89,7 +89,7 @@ static __global__ void __launch_bounds__(256) room_step(RoomArgs<Real> a) {
         st->part[0] = total;
         st->invariant = invariant;
         audit_and_commit(st, total, scale_l);
-    }
+    });
 }
 
 template <typename Real>
@@ -176,7 +176,7 @@ static __global__ void __launch_bounds__(256) tube_step(TubeArgs<Real> a) {
         if (i == 0) acc[1] += fabs(dn * (double)inflow) * a.area * a.dt;
         if (i == n - 1) acc[1] += fabs(dn * (double)outflow) * a.area * a.dt;
     }
-    if (finish_blocks<2>(acc, a.partials, a.nblocks, &st->counter) && linear_tid() == 0) {
+    close_books<2>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double invariant = acc[0];
         if (a.starting) {
             const double off = st->datum - invariant;
@@ -192,7 +192,7 @@ static __global__ void __launch_bounds__(256) tube_step(TubeArgs<Real> a) {
         st->part[1] = st->injected;
         st->invariant = invariant;
         audit_and_commit(st, total, scale_l);
-    }
+    });
 }
 
 template <typename Real>

@@ -774,7 +774,7 @@ static __global__ void __launch_bounds__(256, YeeDepth<Real>::min_blocks) yee_st
         slot = slot + 1 == S ? 0 : slot + 1;
     }
     cp_async_wait<0>();
-    if (finish_blocks<4>(acc, a.partials, a.nblocks, &st->counter) && linear_tid() == 0) {
+    close_books<4>(acc, a.partials, a.nblocks, a.st, [&](DevState* st) {
         const double v = a.volume;
         const double electric = 0.5 * acc[0] * v;   // cavity.rs:846
         const double paired = 0.5 * v * acc[1];     // cavity.rs:885-904
@@ -791,7 +791,7 @@ static __global__ void __launch_bounds__(256, YeeDepth<Real>::min_blocks) yee_st
         st->part[1] = st->dissipated;
         st->part[2] = -st->work_booked;
         audit_and_commit(st, total, scale);
-    }
+    });
 }
 
 // Magnetic and open walls (cavity.rs:1074-1236), applied to the new E after a step, one wall at a

@@ -88,11 +88,10 @@ static __global__ void yee_near_seed(YeeNearArgs a) {
 __device__ __forceinline__ float near_ld_new(const float* p) { return __ldcg(p); }
 
 // Run by the whole last block of yee_tma_step, once every other block's cells are in, with the
-// grid's four sums (valid in thread 0): one work item per (component, node), 3 × w³ in phases A
+// grid's four sums (valid in thread 0) and the books in shared memory: one work item per (component, node), 3 × w³ in phases A
 // and B, 3 × (w+1)³ in phase C, strided over the block's threads.
 template <bool SOLID>
-__device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4]) {
-    DevState* st = a.st;
+__device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4], DevState* st) {
     const int nthreads = blockDim.x * blockDim.y * blockDim.z, tid0 = linear_tid();
     const int w = a.w, w3 = w * w * w;
     const int nx = a.nx, ny = a.ny, nz = a.nz;

@@ -158,10 +158,9 @@ struct YeeNearArgs {
     const double* current;
     long long ncurrent;
     double eps_src, sig_src, dt, volume, g, eps_u, mu_u;
-    DevState* st;
 };
 template <bool SOLID>
-__device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4]);
+__device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4], DevState* st);
 
 // One face of H⁺ (cavity.rs:1346-1379): was − (g/μ)·((a₁ − a₀) − (b₁ − b₀)). The tiles and the
 // wall pass below form every face through this one expression, so the two agree bit for bit.
@@ -437,13 +436,16 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
         }
         return;
     }
-    if (finish_blocks<4>(acc, a.partials, a.nblocks, &st->counter)) {
+    __shared__ DevState books;
+    unsigned long long was = 0;
+    if (last_block<4>(acc, a.partials, a.nblocks, st, books, was)) {
         // the last block: with a near-field box it steps the box, adds the box's terms and closes the
         // books (every other block's cells are in by now: each published its sums after them)
         if (a.nb_w > 0)
-            yee_near_body<SOLID>(nr, acc);
+            yee_near_body<SOLID>(nr, acc, &books);
         else if (linear_tid() == 0)
-            yee_tma_close(st, acc, MEDIA, a.g, a.eps_u, a.mu_u, a.volume, a.src_i >= 0);
+            yee_tma_close(&books, acc, MEDIA, a.g, a.eps_u, a.mu_u, a.volume, a.src_i >= 0);
+        put_books(st, books, was);
     }
 }
 
