@@ -197,7 +197,7 @@ cudaError_t launch_ens_tma(const EnsTmaArgs& t, unsigned nblocks, cudaStream_t s
     const int smem = (int)ens_tma_smem_bytes();
     cudaError_t e = launch_smem(ens_tma_step<kEnsTmaPlanes, kEnsTmaStages>, nblocks, kEnsConsumers + 32, smem, s, t);
     if (e != cudaSuccess) return e;
-    ens_tma_books<<<(t.e.ngrids + 7) / 8, 256, 0, s>>>(t.e);
+    ens_tma_books<<<t.e.ngrids, 256, 0, s>>>(t.e);
     return cudaGetLastError();
 }
 
