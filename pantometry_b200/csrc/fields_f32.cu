@@ -7,9 +7,10 @@
 namespace pm {
 
 cudaError_t launch_heat_f32(const HeatF32Args& a, cudaStream_t s) {
-    if (a.kx) heat_f32_step<true><<<a.nblocks, tile_block(), 0, s>>>(a);
+    if (a.kx) heat_f32_step<true, false><<<a.nblocks, tile_block(), 0, s>>>(a);
     else if (a.quads) heat_f32_quad_step<<<a.nblocks, tile_block(), 0, s>>>(a);
-    else heat_f32_step<false><<<a.nblocks, tile_block(), 0, s>>>(a);
+    else if (a.radiating) heat_f32_step<false, true><<<a.nblocks, tile_block(), 0, s>>>(a);
+    else heat_f32_step<false, false><<<a.nblocks, tile_block(), 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -268,7 +269,9 @@ int occupancy_f32(KernelId id) {
     int n = 0;
     cudaError_t e = cudaSuccess;
     switch (id) {
-        case kHeatF32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_step<false>, 256, 0); break;
+        case kHeatF32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_step<false, false>, 256, 0); break;
+        case kHeatF32Filled: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_step<true, false>, 256, 0); break;
+        case kHeatF32Rad: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_step<false, true>, 256, 0); break;
         case kHeatF32Quad: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_quad_step, 256, 0); break;
         case kHeatF32QuadSteps: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_quad_steps<8>, 256, 0); break;
         case kHeatF32QuadSteps32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_f32_quad_steps<32>, 1024, 0); break;

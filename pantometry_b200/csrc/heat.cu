@@ -467,6 +467,15 @@ struct Heat : Handle {
         a.dts = dt; a.dx = dx; a.reference = reference;
         a.films = films;
         a.films.dirichlet = 0;
+        a.films.plain = 1;
+        for (uint32_t m = 0; m < mats.size(); ++m)
+            if (mat_eps(m) != 0.0) a.films.plain = 0;
+        for (int f = 0; f < 6; ++f) {
+            if (((films.exposed >> f) & 1) && !(std::fabs(films.ambient[f]) < 1e75)) a.films.plain = 0;
+            if (!uniform) continue;
+            a.films.half[f] = 2.0 * mat_k(0) * films.share[f] / dx;  // as series_with_half_cell forms them
+            a.films.inv_half[f] = 1.0 / a.films.half[f];
+        }
         if (uniform) {  // solid.rs:1192-1219 at h = +inf: the film's series with the half cell, per face
             for (int f = 0; f < 6; ++f) {
                 if (!((films.exposed >> f) & 1) || !(films.convection[f] == std::numeric_limits<double>::infinity())) continue;
@@ -475,6 +484,7 @@ struct Heat : Handle {
                                                               films.share[f], dx);
             }
         }
+        a.films.ahead = (films.exposed & ~a.films.dirichlet) != 0 || state_dependent() ? 1 : 0;
         a.quads = uniform && nx % 4 == 0 && wide && quads64 ? 1 : 0;
         a.pairs = !a.quads && uniform && nx % 2 == 0 && wide ? 1 : 0;
         a.radiating = state_dependent() ? 1 : 0;
@@ -547,7 +557,7 @@ struct Heat : Handle {
             a.t0 = reference;
             a.rad = plain_args(par, dt);
         }
-        const unsigned w = wave_of(a.quads ? kHeatF32Quad : kHeatF32);
+        const unsigned w = wave_of(a.quads ? kHeatF32Quad : !uniform ? kHeatF32Filled : a.radiating ? kHeatF32Rad : kHeatF32);
         const int tx = a.quads ? nx / 4 : nx;  // the threads along a row
         a.tiles = make_tiles(tx, ny, nz, choose_zc(tx, ny, nz, w));
         a.nblocks = grid_for(a.tiles, w);

@@ -39,6 +39,14 @@ __device__ __forceinline__ double series_with_half_cell(double film, double cond
     return 1.0 / (1.0 / film + 1.0 / half);
 }
 
+// The same with the half cell's conductance and its inverse at hand.
+__device__ __forceinline__ double series_with_half_cell(double film, double half, double inv_half) {
+    if (film <= 0.0) return 0.0;
+    if (!isfinite(half)) return film;
+    if (half <= 0.0) return 0.0;
+    return 1.0 / (1.0 / film + inv_half);
+}
+
 __device__ __forceinline__ bool face_holds(int f, int i, int j, int k, int nx, int ny, int nz) {
     switch (f) {
         case 0: return i == 0;
@@ -55,6 +63,13 @@ struct HeatFilms {
     double ambient[6];
     double convection[6];
     double share[6];  // area / cells_on(face), computed on the host as the reference does
+    // Blocks of one material: per face the half cell's conductance 2kA/Δx and its inverse, formed once on
+    // the host by series_with_half_cell's own expressions (two of its divisions are the same for every
+    // cell of a face), and whether the material does not radiate and no ambient is so large that a term
+    // of its zero emissivity would not be zero.
+    double half[6], inv_half[6];
+    int plain;
+    int ahead;  // some film is not Dirichlet: films of x and y face cells are formed ahead (HeatFilmCells)
     // Faces with h = +inf on a block of one material: bit f set, and g_inf[f] the film's series
     // with the half cell there, which is the same for every cell of the face (see film_flux).
     int dirichlet;
@@ -139,11 +154,30 @@ __device__ __forceinline__ double film_flux(const HeatPlainArgs& a, int i, int j
         } else {
             // crates/pantometry-thermal/src/lib.rs:104-110 `Environment::loss_from`, area = share
             double convective = a.films.convection[f] * share * (here - ambient);
-            double radiative = emissivity * kStefanBoltzmann * share * (powi4(here) - powi4(ambient));
-            double bare = convective + radiative;
-            g = series_with_half_cell(bare / gap, conductivity, share, a.dx);
+            double bare = convective;
+            // at zero emissivity the radiative term is ±0 wherever here⁴ is finite: it adds nothing
+            if (!(a.films.plain && fabs(here) < 1e75)) {
+                double radiative = emissivity * kStefanBoltzmann * share * (powi4(here) - powi4(ambient));
+                bare = convective + radiative;
+            }
+            g = a.uniform ? series_with_half_cell(bare / gap, a.films.half[f], a.films.inv_half[f])
+                          : series_with_half_cell(bare / gap, conductivity, share, a.dx);
         }
         out += g * gap / a.dx;
+    }
+    return out;
+}
+
+// film_flux where every film is Dirichlet (a block of one material): the face's constant conductance.
+__device__ __forceinline__ double film_flux_dirichlet(const HeatPlainArgs& a, int i, int j, int k, double here) {
+    double out = 0.0;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+        if (!((a.films.exposed >> f) & 1)) continue;
+        if (!face_holds(f, i, j, k, a.nx, a.ny, a.nz)) continue;
+        const double gap = here - a.films.ambient[f];
+        if (gap == 0.0) continue;
+        out += a.films.g_inf[f] * gap / a.dx;
     }
     return out;
 }
@@ -169,7 +203,8 @@ __device__ __forceinline__ double loss_conductance(const HeatPlainArgs& a, int i
         const double share = a.films.share[f];
         const double hot = fmax(at, a.films.ambient[f]);
         const double h = a.films.convection[f] + 4.0 * emissivity * kStefanBoltzmann * powi3(hot);
-        total += series_with_half_cell(h * share, conductivity, share, a.dx);
+        total += a.uniform ? series_with_half_cell(h * share, a.films.half[f], a.films.inv_half[f])
+                           : series_with_half_cell(h * share, conductivity, share, a.dx);
     }
     return total;
 }
@@ -265,6 +300,79 @@ __device__ __forceinline__ double heat_gap_cell(const HeatPlainArgs& a, int g, d
     return nt;
 }
 
+// The films of a tile's cells on x and y faces. A film with a finite conductance is a chain of four
+// divisions or more, tens of times an interior cell's latency, and in the march it falls on the wrong
+// threads: an x face is one lane of each warp, a y face one warp of the block, and every plane waits
+// for it, so the blocks on a face ran long after the others were done. The block therefore forms the
+// films of the tile's face cells side by side into shared memory, kFilmPlanes planes at a time, a cell a
+// thread, and the march reads them there; where the limit follows the state, the march leaves the
+// cells' new temperatures in their place and the block forms their rates the same way. A cell's film is
+// the whole film_flux, all its faces in the order the reference sums them. Cells on z faces only stay in
+// the march: theirs fill every warp of one plane. Dirichlet films (one division) stay in the march too:
+// the barriers cost more (a 64³ block's persistent step ran 5.95 µs in the march, 7.3 with barriers).
+// Measured, µs a step, films in the march and ahead: a radiating 150 × 121 × 93 block of two materials 93.0
+// and 67.0, a convective 256 × 240 × 224 block 135.8 and 113.3, a convective 129 × 111 × 101 one 35.3 and
+// 25.8, a radiating 52 × 41 × 41 one 37.2 and 23.3, FP32 fields on a radiating 160 × 128 × 128 one 42.3 and 32.0.
+constexpr int kFilmPlanes = 8;
+template <int ROWS, int W>
+struct HeatFilmCells {
+    double x[2][ROWS][kFilmPlanes + 1];  // x−, x+ side; row of the tile; plane
+    double y[2][kFilmPlanes][32 * W];    // y−, y+ side; plane; cell along x
+};
+// The tile's place: cells x0 .. x0 + 32·W − 1, rows j0 .. j0 + ROWS − 1, and whether it has cells on x
+// or y faces whose films are formed ahead (uniform in the block, which then takes the barriers).
+struct HeatFilmTile {
+    int x0, j0;
+    bool x, y;
+    __device__ bool any() const { return x || y; }
+};
+template <bool AHEAD, int ROWS, int W>
+__device__ __forceinline__ HeatFilmTile heat_film_tile(const HeatPlainArgs& a, int x0, int j0) {
+    HeatFilmTile t{x0, j0, false, false};
+    if constexpr (AHEAD) {
+        t.x = (a.films.exposed & 3) && (x0 == 0 || x0 + 32 * W >= a.nx);
+        t.y = (a.films.exposed & 12) && (j0 == 0 || j0 + ROWS >= a.ny);
+    }
+    return t;
+}
+// The slot of cell (i, j), plane kk of the present kFilmPlanes, or null where its film is not ahead.
+template <int ROWS, int W>
+__device__ __forceinline__ double* heat_film_slot(HeatFilmCells<ROWS, W>& f, const HeatFilmTile& t, const HeatPlainArgs& a,
+                                                  int i, int j, int kk) {
+    if (t.x && (i == 0 || i + 1 == a.nx)) return &f.x[i == 0 ? 0 : 1][j - t.j0][kk];
+    if (t.y && (j == 0 || j + 1 == a.ny)) return &f.y[j == 0 ? 0 : 1][kk][i - t.x0];
+    return nullptr;
+}
+// Run `one(slot, i, j, k, c)` for every such cell of the tile's planes ka .. kb − 1, over the block.
+template <int ROWS, int W, typename F>
+__device__ __forceinline__ void heat_film_cells(const HeatPlainArgs& a, HeatFilmCells<ROWS, W>& f, const HeatFilmTile& t,
+                                                int ka, int kb, F one) {
+    const int nx = a.nx, ny = a.ny, n = kb - ka;
+    const int xs = t.x ? 2 * ROWS * n : 0, ys = t.y ? 2 * 32 * W * n : 0;
+    for (int r = linear_tid(); r < xs + ys; r += 32 * ROWS) {
+        int i, j, k;
+        double* slot;
+        if (r < xs) {
+            const int side = r >= ROWS * n ? 1 : 0, l = r - side * ROWS * n, kk = l / ROWS, row = l % ROWS;
+            if (side ? (t.x0 + 32 * W < nx || nx == 1) : t.x0 > 0) continue;
+            i = side ? nx - 1 : 0;
+            j = t.j0 + row;
+            k = ka + kk;
+            slot = &f.x[side][row][kk];
+        } else {
+            const int q = r - xs, side = q >= 32 * W * n ? 1 : 0, l = q - side * 32 * W * n, kk = l / (32 * W), col = l % (32 * W);
+            if (side ? (t.j0 + ROWS < ny || ny == 1) : t.j0 > 0) continue;
+            i = t.x0 + col;
+            j = side ? ny - 1 : 0;
+            k = ka + kk;
+            if (t.x && (i == 0 || i + 1 == nx)) continue;  // an x cell's
+            slot = &f.y[side][kk][col];
+        }
+        if (i >= nx || j >= ny) continue;
+        one(*slot, i, j, k, (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * (size_t)k));
+    }
+}
+
 // Decode tile t of a tiling into the thread's column (i, j) and plane range [k0, k1).
 // In 32-bit arithmetic where the tiling allows (a 64-bit division is a long software sequence, and the
 // many-step kernels decode a tile every step).
@@ -318,67 +426,103 @@ __device__ __forceinline__ void heat_plain_books(const HeatPlainArgs& a, double 
 #ifndef PM_HEAT_PLAIN_MIN_BLOCKS
 #define PM_HEAT_PLAIN_MIN_BLOCKS 4
 #endif
+// AHEAD: a.films.ahead, some film that is not Dirichlet, or a limit that follows the state. A kernel of
+// its own, here and for the wide forms below, since the films' divisions, the slots and the rates
+// cost the others their registers (a Dirichlet 256³ block: 107 µs a step with one kernel for all films,
+// 89 here; the 64³ block's persistent step 5.97 and 5.18).
+template <bool AHEAD>
 static __global__ void __launch_bounds__(256, PM_HEAT_PLAIN_MIN_BLOCKS) heat_plain_step(HeatPlainArgs a) {
-    if (a.st->violated || heat_refused(a)) return;
+    if (a.st->violated || (AHEAD && heat_refused(a))) return;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const size_t plane = (size_t)nx * ny;
     double acc[3] = {0.0, 0.0, 0.0};  // stored heat of the new state, heat shed and generated this step
     double rate = -1.0;  // a state-dependent limit: the largest rate of the new state
+    __shared__ HeatFilmCells<8, 1> xf;
     for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x) {
         int i, j, k0, k1;
         tile_column(a.tiles, t, i, j, k0, k1);
-        if (i >= nx || j >= ny) continue;
-        size_t c = (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0);
-        double below = k0 > 0 ? a.told[c - plane] : 0.0;
-        double here = a.told[c];
-        for (int k = k0; k < k1; ++k, c += plane) {
-            const double above = k + 1 < nz ? a.told[c + plane] : 0.0;
-            const double t0 = here;
-            double flux = 0.0;
-            if (a.uniform) {
-                const double kf = a.kface;
-                if (i > 0) flux += kf * (a.told[c - 1] - t0);
-                if (i + 1 < nx) flux += kf * (a.told[c + 1] - t0);
-                if (j > 0) flux += kf * (a.told[c - nx] - t0);
-                if (j + 1 < ny) flux += kf * (a.told[c + nx] - t0);
-                if (k > 0) flux += kf * (below - t0);
-                if (k + 1 < nz) flux += kf * (above - t0);
-            } else {
-                const size_t xr = (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);
-                const size_t yr = (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);
-                if (i > 0) flux += a.kx[i + xr] * (a.told[c - 1] - t0);
-                if (i + 1 < nx) flux += a.kx[i + 1 + xr] * (a.told[c + 1] - t0);
-                if (j > 0) flux += a.ky[i + yr] * (a.told[c - nx] - t0);
-                if (j + 1 < ny) flux += a.ky[i + nx + yr] * (a.told[c + nx] - t0);
-                if (k > 0) flux += a.kz[c] * (below - t0);
-                if (k + 1 < nz) flux += a.kz[c + plane] * (above - t0);
+        const bool live = i < nx && j < ny;
+        const HeatFilmTile ft = heat_film_tile<AHEAD, 8, 1>(a, i - (int)threadIdx.x, j - (int)threadIdx.y);
+        const bool ahead = AHEAD && ft.any();
+        if (!ahead && !live) continue;
+        size_t c = live ? (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0) : 0;
+        double below = live && k0 > 0 ? a.told[c - plane] : 0.0;
+        double here = live ? a.told[c] : 0.0;
+        for (int ka = k0; ka < k1; ka += kFilmPlanes) {
+            const int kb = ahead ? min(k1, ka + kFilmPlanes) : k1;
+            if (ahead) {
+                heat_film_cells(a, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
+                    slot = film_flux(a, fi, fj, fk, fc, a.told[fc]);
+                });
+                __syncthreads();
             }
-            const bool face = i == 0 || i + 1 == nx || j == 0 || j + 1 == ny || k == 0 || k + 1 == nz;
-            const double shed = (a.films.exposed && face) ? film_flux(a, i, j, k, c, t0) : 0.0;
-            const double mob = a.uniform ? a.mobility : a.mob[c];
-            const double capc = a.uniform ? a.capacity : a.cap[c];
-            double nt = t0 + a.dts * mob * (flux - shed);  // add_kelvin, latent <= 0 (solid.rs:1620-1635)
-            if (a.src) {  // solid.rs:1854-1864, after the sweep
-                const double w = a.src[c];
-                if (w != 0.0) {
-                    const double joules = w * a.dts;
-                    nt += joules / capc;
-                    acc[2] += joules;
+            for (int k = live ? ka : kb; k < kb; ++k, c += plane) {
+                const double above = k + 1 < nz ? a.told[c + plane] : 0.0;
+                const double t0 = here;
+                double flux = 0.0;
+                if (a.uniform) {
+                    const double kf = a.kface;
+                    if (i > 0) flux += kf * (a.told[c - 1] - t0);
+                    if (i + 1 < nx) flux += kf * (a.told[c + 1] - t0);
+                    if (j > 0) flux += kf * (a.told[c - nx] - t0);
+                    if (j + 1 < ny) flux += kf * (a.told[c + nx] - t0);
+                    if (k > 0) flux += kf * (below - t0);
+                    if (k + 1 < nz) flux += kf * (above - t0);
+                } else {
+                    const size_t xr = (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);
+                    const size_t yr = (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);
+                    if (i > 0) flux += a.kx[i + xr] * (a.told[c - 1] - t0);
+                    if (i + 1 < nx) flux += a.kx[i + 1 + xr] * (a.told[c + 1] - t0);
+                    if (j > 0) flux += a.ky[i + yr] * (a.told[c - nx] - t0);
+                    if (j + 1 < ny) flux += a.ky[i + nx + yr] * (a.told[c + nx] - t0);
+                    if (k > 0) flux += a.kz[c] * (below - t0);
+                    if (k + 1 < nz) flux += a.kz[c + plane] * (above - t0);
                 }
+                const bool face = i == 0 || i + 1 == nx || j == 0 || j + 1 == ny || k == 0 || k + 1 == nz;
+                double* const slot = ahead ? heat_film_slot(xf, ft, a, i, j, k - ka) : nullptr;
+                double shed = 0.0;
+                if (slot) shed = *slot;
+                else if (a.films.exposed && face)
+                    shed = AHEAD ? film_flux(a, i, j, k, c, t0) : film_flux_dirichlet(a, i, j, k, t0);
+                const double mob = a.uniform ? a.mobility : a.mob[c];
+                const double capc = a.uniform ? a.capacity : a.cap[c];
+                double nt = t0 + a.dts * mob * (flux - shed);  // add_kelvin, latent <= 0 (solid.rs:1620-1635)
+                if (a.src) {  // solid.rs:1854-1864, after the sweep
+                    const double w = a.src[c];
+                    if (w != 0.0) {
+                        const double joules = w * a.dts;
+                        nt += joules / capc;
+                        acc[2] += joules;
+                    }
+                }
+                if (AHEAD && a.gap_of) {
+                    const int g = a.gap_of[c];
+                    if (g >= 0) nt = heat_gap_cell(a, g, t0, capc, nt, rate);
+                }
+                a.tnew[c] = nt;
+                acc[0] += capc * (nt - a.reference);                  // solid.rs:1583-1590
+                if (shed != 0.0) acc[1] += a.dts * mob * shed * capc;  // solid.rs:1821-1823
+                if (AHEAD && a.radiating) {
+                    if (slot) *slot = nt;
+                    else if (face) rate = fmax(rate, heat_cell_rate(a, i, j, k, c, nt));
+                }
+                below = here;
+                here = above;
             }
-            if (a.gap_of) {
-                const int g = a.gap_of[c];
-                if (g >= 0) nt = heat_gap_cell(a, g, t0, capc, nt, rate);
+            if (ahead) {
+                __syncthreads();
+                if (a.radiating) {
+                    heat_film_cells(a, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
+                        rate = fmax(rate, heat_cell_rate(a, fi, fj, fk, fc, slot));
+                    });
+                    __syncthreads();
+                }
+            } else {
+                break;
             }
-            a.tnew[c] = nt;
-            acc[0] += capc * (nt - a.reference);                  // solid.rs:1583-1590
-            if (shed != 0.0) acc[1] += a.dts * mob * shed * capc;  // solid.rs:1821-1823
-            if (a.radiating && face) rate = fmax(rate, heat_cell_rate(a, i, j, k, c, nt));
-            below = here;
-            here = above;
         }
     }
-    if (a.radiating) heat_rate_publish(a, rate);
+    if (AHEAD && a.radiating) heat_rate_publish(a, rate);
     heat_plain_books(a, acc);
 }
 
@@ -411,9 +555,9 @@ __device__ __forceinline__ double heat_ld(const double* p) {
 // One tile of the wide form for one step, from `told` into `tnew`: W adjacent cells of a row per
 // thread (W = 2, the pair form, or 4), the arithmetic the one-step kernels and the persistent
 // many-step kernel run, so they agree bit for bit. Each row of W cells comes in 16-byte loads.
-template <bool CG, int W = 2>
+template <bool CG, int W, int ROWS, bool AHEAD>
 __device__ __forceinline__ void heat_pair_tile(const HeatPlainArgs& a, long long t, const double* told, double* tnew,
-                                               double (&acc)[2], double& rate) {
+                                               double (&acc)[2], double& rate, HeatFilmCells<ROWS, W>& xf) {
     static_assert(W == 2 || W == 4, "two or four cells of a row per thread");
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const size_t plane = (size_t)nx * ny;
@@ -421,8 +565,11 @@ __device__ __forceinline__ void heat_pair_tile(const HeatPlainArgs& a, long long
     int q, j, k0, k1;
     tile_column(a.tiles, t, q, j, k0, k1);  // q: the group's place along the row
     const int i = W * q;
-    if (i >= nx || j >= ny) return;
-    const size_t c0 = (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0);
+    const bool live = i < nx && j < ny;
+    const HeatFilmTile ft = heat_film_tile<AHEAD, ROWS, W>(a, i - W * (int)threadIdx.x, j - (int)threadIdx.y);
+    const bool ahead = AHEAD && ft.any();
+    if (!ahead && !live) return;
+    const size_t c0 = live ? (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0) : 0;
     const double* p = told + c0;
     double* o = tnew + c0;
     const bool xl = i > 0, xh = i + W < nx, yl = j > 0, yh = j + 1 < ny;
@@ -435,68 +582,95 @@ __device__ __forceinline__ void heat_pair_tile(const HeatPlainArgs& a, long long
         }
     };
     double bv[W], hv[W];
-    row(bv, p - plane, k0 > 0);
-    row(hv, p, true);
+    row(bv, p - plane, live && k0 > 0);
+    row(hv, p, live);
     size_t c = c0;
-    for (int k = k0; k < k1; ++k, p += plane, o += plane, c += plane) {
-        double av[W], mv[W], pv[W];
-        row(av, p + plane, k + 1 < nz);
-        row(mv, p - nx, yl);
-        row(pv, p + nx, yh);
-        const double xm = xl ? heat_ld<CG>(p - 1) : 0.0, xp = xh ? heat_ld<CG>(p + W) : 0.0;
-        double nt[W];
-#pragma unroll
-        for (int e = 0; e < W; ++e) {
-            const double t0 = hv[e];
-            double flux = 0.0;
-            if (e > 0 || xl) flux += kf * ((e == 0 ? xm : hv[e > 0 ? e - 1 : 0]) - t0);
-            if (e < W - 1 || xh) flux += kf * ((e == W - 1 ? xp : hv[e + 1 < W ? e + 1 : W - 1]) - t0);
-            if (yl) flux += kf * (mv[e] - t0);
-            if (yh) flux += kf * (pv[e] - t0);
-            if (k > 0) flux += kf * (bv[e] - t0);
-            if (k + 1 < nz) flux += kf * (av[e] - t0);
-            // only a cell on a face can have a film: film_flux is +0 everywhere else
-            const bool face = i + e == 0 || i + e + 1 == nx || !yl || !yh || k == 0 || k + 1 == nz;
-            const double shed = (a.films.exposed && face) ? film_flux(a, i + e, j, k, c + e, t0) : 0.0;
-            nt[e] = t0 + a.dts * a.mobility * (flux - shed);  // add_kelvin, latent <= 0 (solid.rs:1620-1635)
-            acc[0] += a.capacity * (nt[e] - a.reference);     // solid.rs:1583-1590
-            if (shed != 0.0) acc[1] += a.dts * a.mobility * shed * a.capacity;  // solid.rs:1821-1823
-            if (a.radiating && face)
-                rate = fmax(rate, heat_cell_rate(a, i + e, j, k, c + e, nt[e]));
+    for (int ka = k0; ka < k1; ka += kFilmPlanes) {
+        const int kb = ahead ? min(k1, ka + kFilmPlanes) : k1;
+        if (ahead) {
+            heat_film_cells(a, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
+                slot = film_flux(a, fi, fj, fk, fc, heat_ld<CG>(told + fc));
+            });
+            __syncthreads();
         }
+        for (int k = live ? ka : kb; k < kb; ++k, p += plane, o += plane, c += plane) {
+            double av[W], mv[W], pv[W];
+            row(av, p + plane, k + 1 < nz);
+            row(mv, p - nx, yl);
+            row(pv, p + nx, yh);
+            const double xm = xl ? heat_ld<CG>(p - 1) : 0.0, xp = xh ? heat_ld<CG>(p + W) : 0.0;
+            double nt[W];
 #pragma unroll
-        for (int w = 0; w < W / 2; ++w) reinterpret_cast<double2*>(o)[w] = make_double2(nt[2 * w], nt[2 * w + 1]);
+            for (int e = 0; e < W; ++e) {
+                const double t0 = hv[e];
+                double flux = 0.0;
+                if (e > 0 || xl) flux += kf * ((e == 0 ? xm : hv[e > 0 ? e - 1 : 0]) - t0);
+                if (e < W - 1 || xh) flux += kf * ((e == W - 1 ? xp : hv[e + 1 < W ? e + 1 : W - 1]) - t0);
+                if (yl) flux += kf * (mv[e] - t0);
+                if (yh) flux += kf * (pv[e] - t0);
+                if (k > 0) flux += kf * (bv[e] - t0);
+                if (k + 1 < nz) flux += kf * (av[e] - t0);
+                // only a cell on a face can have a film: film_flux is +0 everywhere else
+                const bool face = i + e == 0 || i + e + 1 == nx || !yl || !yh || k == 0 || k + 1 == nz;
+                double* const slot = ahead ? heat_film_slot(xf, ft, a, i + e, j, k - ka) : nullptr;
+                double shed = 0.0;
+                if (slot) shed = *slot;
+                else if (a.films.exposed && face)
+                    shed = AHEAD ? film_flux(a, i + e, j, k, c + e, t0) : film_flux_dirichlet(a, i + e, j, k, t0);
+                nt[e] = t0 + a.dts * a.mobility * (flux - shed);  // add_kelvin, latent <= 0 (solid.rs:1620-1635)
+                acc[0] += a.capacity * (nt[e] - a.reference);     // solid.rs:1583-1590
+                if (shed != 0.0) acc[1] += a.dts * a.mobility * shed * a.capacity;  // solid.rs:1821-1823
+                if (AHEAD && a.radiating) {
+                    if (slot) *slot = nt[e];
+                    else if (face) rate = fmax(rate, heat_cell_rate(a, i + e, j, k, c + e, nt[e]));
+                }
+            }
 #pragma unroll
-        for (int e = 0; e < W; ++e) {
-            bv[e] = hv[e];
-            hv[e] = av[e];
+            for (int w = 0; w < W / 2; ++w) reinterpret_cast<double2*>(o)[w] = make_double2(nt[2 * w], nt[2 * w + 1]);
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                bv[e] = hv[e];
+                hv[e] = av[e];
+            }
+        }
+        if (!ahead) break;
+        __syncthreads();
+        if (a.radiating) {
+            heat_film_cells(a, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
+                rate = fmax(rate, heat_cell_rate(a, fi, fj, fk, fc, slot));
+            });
+            __syncthreads();
         }
     }
 }
 
+template <bool AHEAD>
 static __global__ void __launch_bounds__(256, PM_HEAT_PAIR_MIN_BLOCKS) heat_plain_pair_step(HeatPlainArgs a) {
-    if (a.st->violated || heat_refused(a)) return;
+    if (a.st->violated || (AHEAD && heat_refused(a))) return;
     double acc[2] = {0.0, 0.0};  // stored heat of the new state, heat shed this step
     double rate = -1.0;  // a state-dependent limit: the largest rate of the new state
-    for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x) heat_pair_tile<false>(a, t, a.told, a.tnew, acc, rate);
-    if (a.radiating) heat_rate_publish(a, rate);
+    __shared__ HeatFilmCells<8, 2> xf;
+    for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x)
+        heat_pair_tile<false, 2, 8, AHEAD>(a, t, a.told, a.tnew, acc, rate, xf);
+    if (AHEAD && a.radiating) heat_rate_publish(a, rate);
     heat_plain_books(a, acc);
 }
 
 // Four cells of a row per thread (rows of a multiple of 4 cells): four independent FP64 chains a
-// thread, where the reference's sequential flux sum makes each cell one chain. Measured on a 256³
-// block: 170 Gcell/s at two blocks of 256 per SM (no bound on registers), 159 at three (80
-// registers, a few bytes spilled), against the pair form's 161.
+// thread, where the reference's sequential flux sum makes each cell one chain. Measured on a
+// Dirichlet 256³ block: 188 Gcell/s at two blocks of 256 per SM (96 registers).
 #ifndef PM_HEAT_QUAD64_MIN_BLOCKS
 #define PM_HEAT_QUAD64_MIN_BLOCKS 2
 #endif
+template <bool AHEAD>
 static __global__ void __launch_bounds__(256, PM_HEAT_QUAD64_MIN_BLOCKS) heat_plain_quad_step(HeatPlainArgs a) {
-    if (a.st->violated || heat_refused(a)) return;
+    if (a.st->violated || (AHEAD && heat_refused(a))) return;
     double acc[2] = {0.0, 0.0};  // stored heat of the new state, heat shed this step
     double rate = -1.0;  // a state-dependent limit: the largest rate of the new state
+    __shared__ HeatFilmCells<8, 4> xf;
     for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x)
-        heat_pair_tile<false, 4>(a, t, a.told, a.tnew, acc, rate);
-    if (a.radiating) heat_rate_publish(a, rate);
+        heat_pair_tile<false, 4, 8, AHEAD>(a, t, a.told, a.tnew, acc, rate, xf);
+    if (AHEAD && a.radiating) heat_rate_publish(a, rate);
     heat_plain_books(a, acc);
 }
 
@@ -595,14 +769,15 @@ __device__ __forceinline__ void heat_persist(const Args& a, const HeatPersist& p
 
 // The pair form's many-step kernel: blocks of 32 × ROWS threads (8 rows: four blocks per SM; 32 rows:
 // one block of 1024 per SM, so a 64³ block is 128 workers and the keeper).
-template <int ROWS>
+template <int ROWS, bool AHEAD>
 static __global__ void __launch_bounds__(32 * ROWS, ROWS == 8 ? PM_HEAT_PAIR_MIN_BLOCKS : 1)
     heat_plain_pair_steps(HeatPlainArgs a, HeatPersist p) {
+    __shared__ HeatFilmCells<ROWS, 2> xf;
     heat_persist(a, p, 1.0, [&](int s, long long first, long long stride, double (&acc)[2]) {
         const double* told = (s & 1) ? a.tnew : a.told;
         double* tnew = const_cast<double*>((s & 1) ? a.told : a.tnew);
         double rate = -1.0;
-        for (long long t = first; t < a.tiles.ntiles; t += stride) heat_pair_tile<true>(a, t, told, tnew, acc, rate);
+        for (long long t = first; t < a.tiles.ntiles; t += stride) heat_pair_tile<true, 2, ROWS, AHEAD>(a, t, told, tnew, acc, rate, xf);
     });
 }
 
@@ -665,98 +840,122 @@ __device__ __forceinline__ void heat_f32_books(const HeatF32Args& a, double (&ac
 }
 
 // Chosen form, z-marching like the plain form; neighbours in the plane come from L1/L2.
-template <bool FILLED>
-static __global__ void __launch_bounds__(256) heat_f32_step(HeatF32Args a) {
-    if (a.st->violated || (a.radiating && heat_refused(a.rad))) return;
+// RAD: a.radiating, a uniform block whose films radiate (held to four blocks per SM; the films' code
+// would take the kernel to two).
+template <bool FILLED, bool RAD>
+static __global__ void __launch_bounds__(256, RAD ? 4 : 1) heat_f32_step(HeatF32Args a) {
+    if (a.st->violated || (RAD && heat_refused(a.rad))) return;
     double rate = -1.0;  // radiating films: the largest rate of the new state
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const size_t plane = (size_t)nx * ny;
     double acc[FILLED ? 3 : 2] = {};
+    __shared__ HeatFilmCells<8, 1> xf;
     for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x) {
         int i, j, k0, k1;
         tile_column(a.tiles, t, i, j, k0, k1);
-        if (i >= nx || j >= ny) continue;
-        size_t c = (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0);
-        float below = k0 > 0 ? __ldg(a.dold + c - plane) : 0.0f;
-        float here = __ldg(a.dold + c);
+        const bool live = i < nx && j < ny;
+        const HeatFilmTile ft = heat_film_tile<RAD, 8, 1>(a.rad, i - (int)threadIdx.x, j - (int)threadIdx.y);
+        const bool ahead = RAD && ft.any();
+        if (!ahead && !live) continue;
+        size_t c = live ? (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0) : 0;
+        float below = live && k0 > 0 ? __ldg(a.dold + c - plane) : 0.0f;
+        float here = live ? __ldg(a.dold + c) : 0.0f;
         const bool xl = i > 0, xh = i + 1 < nx, yl = j > 0, yh = j + 1 < ny;
         const bool edge_xy = !(xl && xh && yl && yh);
         double col_shed = 0.0;
-        for (int k = k0; k < k1; ++k, c += plane) {
-            const float above = (k + 1 < nz) ? __ldg(a.dold + c + plane) : 0.0f;
-            float s = 0.0f;
-            if constexpr (FILLED) {
-                // solid.rs:1773-1826 in the reference's arm order, each face's own conductivity
-                const size_t xr = (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);
-                const size_t yr = (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);
-                if (xl) s += __ldg(a.kx + i + xr) * (__ldg(a.dold + c - 1) - here);
-                if (xh) s += __ldg(a.kx + i + 1 + xr) * (__ldg(a.dold + c + 1) - here);
-                if (yl) s += __ldg(a.ky + i + yr) * (__ldg(a.dold + c - nx) - here);
-                if (yh) s += __ldg(a.ky + i + nx + yr) * (__ldg(a.dold + c + nx) - here);
-                if (k > 0) s += __ldg(a.kz + c) * (below - here);
-                if (k + 1 < nz) s += __ldg(a.kz + c + plane) * (above - here);
-            } else {
-                if (xl) s += __ldg(a.dold + c - 1) - here;
-                if (xh) s += __ldg(a.dold + c + 1) - here;
-                if (yl) s += __ldg(a.dold + c - nx) - here;
-                if (yh) s += __ldg(a.dold + c + nx) - here;
-                if (k > 0) s += below - here;
-                if (k + 1 < nz) s += above - here;
+        for (int ka = k0; ka < k1; ka += kFilmPlanes) {
+            const int kb = ahead ? min(k1, ka + kFilmPlanes) : k1;
+            if (ahead) {
+                heat_film_cells(a.rad, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
+                    slot = film_flux(a.rad, fi, fj, fk, fc, a.t0 + (double)__ldg(a.dold + fc));
+                });
+                __syncthreads();
             }
-            float shed = 0.0f;
-            if (a.exposed && (edge_xy || k == 0 || k + 1 == nz)) {
+            for (int k = live ? ka : kb; k < kb; ++k, c += plane) {
+                const float above = (k + 1 < nz) ? __ldg(a.dold + c + plane) : 0.0f;
+                float s = 0.0f;
                 if constexpr (FILLED) {
-                    const unsigned px = (unsigned)j + (unsigned)ny * (unsigned)k, py = (unsigned)i + (unsigned)nx * (unsigned)k,
-                                   pz = (unsigned)i + (unsigned)nx * (unsigned)j;
-                    if (((a.exposed >> 0) & 1) && !xl) shed += __ldg(a.film[0] + px) * (here + a.off[0]);
-                    if (((a.exposed >> 1) & 1) && !xh) shed += __ldg(a.film[1] + px) * (here + a.off[1]);
-                    if (((a.exposed >> 2) & 1) && !yl) shed += __ldg(a.film[2] + py) * (here + a.off[2]);
-                    if (((a.exposed >> 3) & 1) && !yh) shed += __ldg(a.film[3] + py) * (here + a.off[3]);
-                    if (((a.exposed >> 4) & 1) && k == 0) shed += __ldg(a.film[4] + pz) * (here + a.off[4]);
-                    if (((a.exposed >> 5) & 1) && k + 1 == nz) shed += __ldg(a.film[5] + pz) * (here + a.off[5]);
-                } else if (a.radiating) {
-                    // solid.rs:1192-1219 at the cell's kelvin, as dt · mobility · flux
-                    shed = (float)(a.rad.dts * a.rad.mobility * film_flux(a.rad, i, j, k, c, a.t0 + (double)here));
-                    col_shed += (double)shed;
+                    // solid.rs:1773-1826 in the reference's arm order, each face's own conductivity
+                    const size_t xr = (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);
+                    const size_t yr = (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);
+                    if (xl) s += __ldg(a.kx + i + xr) * (__ldg(a.dold + c - 1) - here);
+                    if (xh) s += __ldg(a.kx + i + 1 + xr) * (__ldg(a.dold + c + 1) - here);
+                    if (yl) s += __ldg(a.ky + i + yr) * (__ldg(a.dold + c - nx) - here);
+                    if (yh) s += __ldg(a.ky + i + nx + yr) * (__ldg(a.dold + c + nx) - here);
+                    if (k > 0) s += __ldg(a.kz + c) * (below - here);
+                    if (k + 1 < nz) s += __ldg(a.kz + c + plane) * (above - here);
                 } else {
-                    if (((a.exposed >> 0) & 1) && !xl) shed += a.b[0] * (here + a.off[0]);
-                    if (((a.exposed >> 1) & 1) && !xh) shed += a.b[1] * (here + a.off[1]);
-                    if (((a.exposed >> 2) & 1) && !yl) shed += a.b[2] * (here + a.off[2]);
-                    if (((a.exposed >> 3) & 1) && !yh) shed += a.b[3] * (here + a.off[3]);
-                    if (((a.exposed >> 4) & 1) && k == 0) shed += a.b[4] * (here + a.off[4]);
-                    if (((a.exposed >> 5) & 1) && k + 1 == nz) shed += a.b[5] * (here + a.off[5]);
-                    col_shed += (double)shed;
+                    if (xl) s += __ldg(a.dold + c - 1) - here;
+                    if (xh) s += __ldg(a.dold + c + 1) - here;
+                    if (yl) s += __ldg(a.dold + c - nx) - here;
+                    if (yh) s += __ldg(a.dold + c + nx) - here;
+                    if (k > 0) s += below - here;
+                    if (k + 1 < nz) s += above - here;
                 }
-            }
-            float nd;
-            if constexpr (FILLED) {
-                // add_kelvin (solid.rs:1620-1635); stored heat C·dev and shed heat C·dt·mob·shed
-                const float mc = __ldg(a.m + c);
-                nd = here + mc * (s - shed);
-                const double capc = __ldg(a.cap + c);
-                if (a.src) {  // solid.rs:1854-1864, after the sweep: the joules in FP64, the rise in f32
-                    const double w = __ldg(a.src + c);
-                    if (w != 0.0) {
-                        const double joules = w * a.dts;
-                        nd += (float)(joules / capc);
-                        acc[FILLED ? 2 : 0] += joules;
+                double* const slot = ahead ? heat_film_slot(xf, ft, a.rad, i, j, k - ka) : nullptr;
+                float shed = 0.0f;
+                if (a.exposed && (edge_xy || k == 0 || k + 1 == nz)) {
+                    if constexpr (FILLED) {
+                        const unsigned px = (unsigned)j + (unsigned)ny * (unsigned)k, py = (unsigned)i + (unsigned)nx * (unsigned)k,
+                                       pz = (unsigned)i + (unsigned)nx * (unsigned)j;
+                        if (((a.exposed >> 0) & 1) && !xl) shed += __ldg(a.film[0] + px) * (here + a.off[0]);
+                        if (((a.exposed >> 1) & 1) && !xh) shed += __ldg(a.film[1] + px) * (here + a.off[1]);
+                        if (((a.exposed >> 2) & 1) && !yl) shed += __ldg(a.film[2] + py) * (here + a.off[2]);
+                        if (((a.exposed >> 3) & 1) && !yh) shed += __ldg(a.film[3] + py) * (here + a.off[3]);
+                        if (((a.exposed >> 4) & 1) && k == 0) shed += __ldg(a.film[4] + pz) * (here + a.off[4]);
+                        if (((a.exposed >> 5) & 1) && k + 1 == nz) shed += __ldg(a.film[5] + pz) * (here + a.off[5]);
+                    } else if constexpr (RAD) {
+                        // solid.rs:1192-1219 at the cell's kelvin, as dt · mobility · flux
+                        const double flux = slot ? *slot : film_flux(a.rad, i, j, k, c, a.t0 + (double)here);
+                        shed = (float)(a.rad.dts * a.rad.mobility * flux);
+                        col_shed += (double)shed;
+                    } else {
+                        if (((a.exposed >> 0) & 1) && !xl) shed += a.b[0] * (here + a.off[0]);
+                        if (((a.exposed >> 1) & 1) && !xh) shed += a.b[1] * (here + a.off[1]);
+                        if (((a.exposed >> 2) & 1) && !yl) shed += a.b[2] * (here + a.off[2]);
+                        if (((a.exposed >> 3) & 1) && !yh) shed += a.b[3] * (here + a.off[3]);
+                        if (((a.exposed >> 4) & 1) && k == 0) shed += a.b[4] * (here + a.off[4]);
+                        if (((a.exposed >> 5) & 1) && k + 1 == nz) shed += a.b[5] * (here + a.off[5]);
+                        col_shed += (double)shed;
                     }
                 }
-                acc[0] += capc * (double)nd;
-                if (shed != 0.0f) acc[1] += capc * (double)(mc * shed);
-            } else {
-                nd = here + (a.a * s - shed);
-                acc[0] += (double)nd;
-                if (a.radiating && (edge_xy || k == 0 || k + 1 == nz))
-                    rate = fmax(rate, heat_cell_rate(a.rad, i, j, k, c, a.t0 + (double)nd));
+                float nd;
+                if constexpr (FILLED) {
+                    // add_kelvin (solid.rs:1620-1635); stored heat C·dev and shed heat C·dt·mob·shed
+                    const float mc = __ldg(a.m + c);
+                    nd = here + mc * (s - shed);
+                    const double capc = __ldg(a.cap + c);
+                    if (a.src) {  // solid.rs:1854-1864, after the sweep: the joules in FP64, the rise in f32
+                        const double w = __ldg(a.src + c);
+                        if (w != 0.0) {
+                            const double joules = w * a.dts;
+                            nd += (float)(joules / capc);
+                            acc[FILLED ? 2 : 0] += joules;
+                        }
+                    }
+                    acc[0] += capc * (double)nd;
+                    if (shed != 0.0f) acc[1] += capc * (double)(mc * shed);
+                } else {
+                    nd = here + (a.a * s - shed);
+                    acc[0] += (double)nd;
+                    if (slot) *slot = a.t0 + (double)nd;
+                    else if (RAD && (edge_xy || k == 0 || k + 1 == nz))
+                        rate = fmax(rate, heat_cell_rate(a.rad, i, j, k, c, a.t0 + (double)nd));
+                }
+                a.dnew[c] = nd;
+                below = here;
+                here = above;
             }
-            a.dnew[c] = nd;
-            below = here;
-            here = above;
+            if (!ahead) break;
+            __syncthreads();
+            heat_film_cells(a.rad, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
+                rate = fmax(rate, heat_cell_rate(a.rad, fi, fj, fk, fc, slot));
+            });
+            __syncthreads();
         }
         acc[1] += col_shed;
     }
-    if (a.radiating) heat_rate_publish(a.rad, rate);
+    if (RAD) heat_rate_publish(a.rad, rate);
     heat_f32_books(a, acc, FILLED);
 }
 

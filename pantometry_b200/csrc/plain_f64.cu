@@ -7,9 +7,11 @@
 namespace pm {
 
 cudaError_t launch_heat_plain(const HeatPlainArgs& a, cudaStream_t s) {
-    if (a.quads) heat_plain_quad_step<<<a.nblocks, tile_block(), 0, s>>>(a);
-    else if (a.pairs) heat_plain_pair_step<<<a.nblocks, tile_block(), 0, s>>>(a);
-    else heat_plain_step<<<a.nblocks, tile_block(), 0, s>>>(a);
+    const bool ahead = a.films.ahead != 0;
+    auto k = a.quads   ? (ahead ? heat_plain_quad_step<true> : heat_plain_quad_step<false>)
+             : a.pairs ? (ahead ? heat_plain_pair_step<true> : heat_plain_pair_step<false>)
+                       : (ahead ? heat_plain_step<true> : heat_plain_step<false>);
+    k<<<a.nblocks, tile_block(), 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -18,10 +20,10 @@ cudaError_t launch_heat_plain_steps(const HeatPlainArgs& a, const HeatPersist& p
     HeatPersist pp = p;
     void* args[2] = {&aa, &pp};
     // the tiling's rows are the block's y extent: 8 (256 threads) or 32 (1024)
-    if (a.tiles.rows == 32)
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(heat_plain_pair_steps<32>), dim3(a.nblocks),
-                                           dim3(32, 32), args, 0, s);
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(heat_plain_pair_steps<8>), dim3(a.nblocks), tile_block(),
+    const bool tall = a.tiles.rows == 32, ahead = a.films.ahead != 0;
+    auto k = tall ? (ahead ? heat_plain_pair_steps<32, true> : heat_plain_pair_steps<32, false>)
+                  : (ahead ? heat_plain_pair_steps<8, true> : heat_plain_pair_steps<8, false>);
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(a.nblocks), tall ? dim3(32, 32) : tile_block(),
                                        args, 0, s);
 }
 
@@ -188,11 +190,11 @@ int occupancy_f64(KernelId id) {
     int n = 0;
     cudaError_t e = cudaSuccess;
     switch (id) {
-        case kHeatPlain: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_step, 256, 0); break;
-        case kHeatPlainPair: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_step, 256, 0); break;
-        case kHeatPlainQuad: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_quad_step, 256, 0); break;
-        case kHeatPlainSteps: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<8>, 256, 0); break;
-        case kHeatPlainSteps32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<32>, 1024, 0); break;
+        case kHeatPlain: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_step<true>, 256, 0); break;
+        case kHeatPlainPair: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_step<true>, 256, 0); break;
+        case kHeatPlainQuad: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_quad_step<true>, 256, 0); break;
+        case kHeatPlainSteps: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<8, true>, 256, 0); break;
+        case kHeatPlainSteps32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<32, true>, 1024, 0); break;
         case kHallF64:
             e = allow_smem(hall_step<double, false>, (int)hall_smem_bytes<double>());
             if (e != cudaSuccess) break;
