@@ -690,19 +690,7 @@ struct Cavity : Handle {
         const bool src_on_wall = a.src_i >= 0 && (a.src_i == nx || a.src_j == ny);
         a.wall_split = (wall_split_on && nx % 32 == 0 && ny % 8 == 0 && !src_on_wall) ? 1 : 0;
         const int X = a.wall_split ? nx : nx + 1, Y = a.wall_split ? ny : ny + 1, Z = nz + 1;
-        int best = 2 * P - 1;
-        double best_score = -1.0;
-        for (int mlt : {2, 4, 8, 16}) {
-            const int zc = P * mlt - 1;
-            if (zc > Z && zc != 2 * P - 1) continue;
-            const Tiles t = make_tiles(X, Y, Z, zc);
-            const double per = (double)t.ntiles / w;
-            const double rounds = per < 1.0 ? 1.0 : (double)((t.ntiles + w - 1) / w);
-            const double balance = per < 1.0 ? per : per / rounds;
-            const double score = balance * (1.0 - 1.0 / (2.0 * zc));
-            if (score > best_score + 1e-9) { best_score = score; best = zc; }
-        }
-        a.tiles = make_tiles(X, Y, Z, best);
+        a.tiles = make_tiles(X, Y, Z, choose_zc(X, Y, Z, w, P, 1));
         a.nblocks = grid_for(a.tiles, w);
         return a;
     }

@@ -108,7 +108,7 @@ extern "C" pm_status pm_hall_step_f32_noalloc(int nx, int ny, int nz, double dx,
     a.src = -1;
     a.src_i = a.src_j = a.src_k = -1;
     a.starting = 0;
-    a.tiles = make_tiles(nx, ny, nz, choose_zc(nx, ny, nz, (unsigned)d.wave));
+    a.tiles = make_tiles(nx, ny, nz, choose_zc(nx, ny, nz, (unsigned)d.wave, 2));
     a.nblocks = grid_for(a.tiles, (unsigned)d.wave);
     // scratch layout: the state block, then 3 partial sums per block
     const size_t state_bytes = (sizeof(DevState) + 255) & ~size_t(255);
