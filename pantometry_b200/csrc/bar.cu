@@ -81,10 +81,17 @@ struct Bar : Handle {
 
 using namespace pm;
 
-#define BAR_GUARD(b)                                          \
+// Entry of a call that reads the handle or steps it (LOOK), and of every other (GUARD), which may
+// change the state block behind its mirror.
+#define BAR_LOOK(b)                                          \
     do {                                                      \
         if (!(b)) return fail(PM_BAD_ARG, "null pm_bar");      \
         cudaSetDevice((b)->device);                           \
+    } while (0)
+#define BAR_GUARD(b) \
+    do {               \
+        BAR_LOOK(b);  \
+        (b)->mirror = false; \
     } while (0)
 
 extern "C" {
@@ -132,7 +139,7 @@ pm_status pm_bar_upload(pm_bar* bp, const double* kelvin, size_t n) {
 
 pm_status pm_bar_download(pm_bar* bp, double* kelvin, size_t n) {
     Bar* b = reinterpret_cast<Bar*>(bp);
-    BAR_GUARD(b);
+    BAR_LOOK(b);
     if (!kelvin || n != (size_t)b->n) return fail(PM_BAD_ARG, "download: one temperature per cell");
     if (b->precision == PM_PLAIN_F64) {
         PM_CUDA(cudaMemcpyAsync(kelvin, b->field[b->parity].p, n * 8, cudaMemcpyDeviceToHost, b->stream()));
@@ -147,7 +154,7 @@ pm_status pm_bar_download(pm_bar* bp, double* kelvin, size_t n) {
 
 pm_status pm_bar_sample(pm_bar* bp, const double* lo, const double* hi, const int* samples, double* out, size_t n) {
     Bar* b = reinterpret_cast<Bar*>(bp);
-    BAR_GUARD(b);
+    BAR_LOOK(b);
     SampleGrid g{};
     pm_status s = sample_grid_of(lo, hi, samples, out, n, g);
     if (s != PM_OK) return s;
@@ -178,7 +185,7 @@ pm_status pm_bar_deposit(pm_bar* bp, const double* joules, size_t n) {
 
 pm_status pm_bar_max_stable_dt(pm_bar* bp, double* seconds) {
     Bar* b = reinterpret_cast<Bar*>(bp);
-    BAR_GUARD(b);
+    BAR_LOOK(b);
     if (!seconds) return fail(PM_BAD_ARG, "null output");
     // lib.rs:564-569
     *seconds = b->sub.thermal ? b->dx * b->dx / (2.0 * b->diffusivity()) : std::numeric_limits<double>::infinity();
@@ -187,14 +194,14 @@ pm_status pm_bar_max_stable_dt(pm_bar* bp, double* seconds) {
 
 pm_status pm_bar_set_tolerance(pm_bar* bp, double tol) {
     Bar* b = reinterpret_cast<Bar*>(bp);
-    BAR_GUARD(b);
+    BAR_LOOK(b);
     b->tolerance = tol;
     return PM_OK;
 }
 
 pm_status pm_bar_step(pm_bar* bp, double dt, long long nsteps, pm_violation* out) {
     Bar* b = reinterpret_cast<Bar*>(bp);
-    BAR_GUARD(b);
+    BAR_LOOK(b);
     if (nsteps < 0) return fail(PM_BAD_ARG, "nsteps must be >= 0");
     if (nsteps == 0) return PM_OK;
     // lib.rs:571-589
@@ -242,9 +249,9 @@ pm_status pm_bar_step(pm_bar* bp, double dt, long long nsteps, pm_violation* out
 
 pm_status pm_bar_ledger(pm_bar* bp, pm_ledger* out) {
     Bar* b = reinterpret_cast<Bar*>(bp);
-    BAR_GUARD(b);
+    BAR_LOOK(b);
     if (!out) return fail(PM_BAD_ARG, "null output");
-    pm_status s = b->read_state();
+    pm_status s = b->latest_state();
     if (s != PM_OK) return s;
     std::memset(out, 0, sizeof(*out));
     const DevState* st = b->host_state;

@@ -802,10 +802,17 @@ struct Cavity : Handle {
 
 using namespace pm;
 
-#define CAV_GUARD(c)                                            \
+// Entry of a call that reads the handle or steps it (LOOK), and of every other (GUARD), which may
+// change the state block behind its mirror.
+#define CAV_LOOK(c)                                            \
     do {                                                        \
         if (!(c)) return fail(PM_BAD_ARG, "null pm_cavity");     \
         cudaSetDevice((c)->device);                             \
+    } while (0)
+#define CAV_GUARD(c) \
+    do {               \
+        CAV_LOOK(c);  \
+        (c)->mirror = false; \
     } while (0)
 
 extern "C" {
@@ -942,7 +949,7 @@ pm_status pm_cavity_upload(pm_cavity* cp, const double* ex, const double* ey, co
 
 pm_status pm_cavity_download(pm_cavity* cp, double* ex, double* ey, double* ez, double* hx, double* hy, double* hz) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     double* dst[6] = {ex, ey, ez, hx, hy, hz};
     pm_status s;
     for (int q = 0; q < 6; ++q)
@@ -1025,7 +1032,7 @@ pm_status pm_cavity_set_source(pm_cavity* cp, long long edge, const double* cur,
 
 pm_status pm_cavity_courant_limit(pm_cavity* cp, double* seconds) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     if (!seconds) return fail(PM_BAD_ARG, "null output");
     *seconds = c->courant_limit();
     return PM_OK;
@@ -1033,14 +1040,14 @@ pm_status pm_cavity_courant_limit(pm_cavity* cp, double* seconds) {
 
 pm_status pm_cavity_set_tolerance(pm_cavity* cp, double tol) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     c->tolerance = tol;
     return PM_OK;
 }
 
 pm_status pm_cavity_step(pm_cavity* cp, double dt, long long nsteps, pm_violation* out) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     if (nsteps < 0) return fail(PM_BAD_ARG, "nsteps must be >= 0");
     if (nsteps == 0) return PM_OK;
     if (c->solid_after_walls()) {
@@ -1089,9 +1096,9 @@ pm_status pm_cavity_step(pm_cavity* cp, double dt, long long nsteps, pm_violatio
 
 pm_status pm_cavity_ledger(pm_cavity* cp, pm_ledger* out) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     if (!out) return fail(PM_BAD_ARG, "null output");
-    pm_status s = c->read_state();
+    pm_status s = c->latest_state();
     if (s != PM_OK) return s;
     std::memset(out, 0, sizeof(*out));
     const DevState* st = c->host_state;
@@ -1108,7 +1115,7 @@ pm_status pm_cavity_ledger(pm_cavity* cp, pm_ledger* out) {
 pm_status pm_cavity_sample(pm_cavity* cp, const double* lo, const double* hi, const int* samples, double* out,
                            size_t n) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     SampleGrid g{};
     pm_status s = sample_grid_of(lo, hi, samples, out, n, g);
     if (s != PM_OK) return s;
@@ -1209,7 +1216,7 @@ pm_status pm_cavity_set_tile(pm_cavity* cp, int planes, int stages) {
 
 pm_status pm_cavity_tile(pm_cavity* cp, int* planes, int* stages) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     const YeeTmaShape sh = yee_tma_shape(!c->uniform, c->yshape);
     if (planes) *planes = c->tma ? sh.planes : 0;
     if (stages) *stages = c->tma ? sh.stages : 0;
@@ -1228,7 +1235,7 @@ pm_status pm_cavity_set_wall_split(pm_cavity* cp, int on) {
 
 pm_status pm_cavity_wall_split(pm_cavity* cp, int* on) {
     Cavity* c = reinterpret_cast<Cavity*>(cp);
-    CAV_GUARD(c);
+    CAV_LOOK(c);
     if (on) *on = (c->tma && c->targs(c->parity, c->courant_limit()).wall_split) ? 1 : 0;
     return PM_OK;
 }

@@ -306,10 +306,17 @@ struct Hall : Handle {
 
 using namespace pm;
 
-#define HALL_GUARD(h)                                          \
+// Entry of a call that reads the handle or steps it (LOOK), and of every other (GUARD), which may
+// change the state block behind its mirror.
+#define HALL_LOOK(h)                                          \
     do {                                                       \
         if (!(h)) return fail(PM_BAD_ARG, "null pm_hall");      \
         cudaSetDevice((h)->device);                            \
+    } while (0)
+#define HALL_GUARD(h) \
+    do {               \
+        HALL_LOOK(h);  \
+        (h)->mirror = false; \
     } while (0)
 
 extern "C" {
@@ -358,7 +365,7 @@ pm_status pm_hall_create(const pm_hall_desc* d, pm_hall** out) {
 
 pm_status pm_hall_nodes(pm_hall* hp, int* nx, int* ny, int* nz, double* dx) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     if (nx) *nx = h->nx;
     if (ny) *ny = h->ny;
     if (nz) *nz = h->nz;
@@ -444,7 +451,7 @@ pm_status pm_hall_set_speed_blocks(pm_hall* hp, int block, const double* speeds,
 
 pm_status pm_hall_max_stable_dt(pm_hall* hp, double* seconds) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     if (!seconds) return fail(PM_BAD_ARG, "null output");
     // hall.rs:401-406 (with the fastest block when the speed varies)
     const double c = h->block > 0 ? h->max_speed : h->speed;
@@ -454,14 +461,14 @@ pm_status pm_hall_max_stable_dt(pm_hall* hp, double* seconds) {
 
 pm_status pm_hall_set_tolerance(pm_hall* hp, double tol) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     h->tolerance = tol;
     return PM_OK;
 }
 
 pm_status pm_hall_step(pm_hall* hp, double dt, long long nsteps, pm_violation* out) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     if (nsteps < 0) return fail(PM_BAD_ARG, "nsteps must be >= 0");
     if (nsteps == 0) return PM_OK;
     // hall.rs:409-419
@@ -492,9 +499,9 @@ pm_status pm_hall_step(pm_hall* hp, double dt, long long nsteps, pm_violation* o
 
 pm_status pm_hall_ledger(pm_hall* hp, pm_ledger* out) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     if (!out) return fail(PM_BAD_ARG, "null output");
-    pm_status s = h->read_state();
+    pm_status s = h->latest_state();
     if (s != PM_OK) return s;
     std::memset(out, 0, sizeof(*out));
     const DevState* st = h->host_state;
@@ -511,7 +518,7 @@ pm_status pm_hall_ledger(pm_hall* hp, pm_ledger* out) {
 
 pm_status pm_hall_sample(pm_hall* hp, const double* lo, const double* hi, const int* samples, double* out, size_t n) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     SampleGrid g{};
     pm_status s = sample_grid_of(lo, hi, samples, out, n, g);
     if (s != PM_OK) return s;
@@ -525,7 +532,7 @@ pm_status pm_hall_sample(pm_hall* hp, const double* lo, const double* hi, const 
 
 pm_status pm_hall_download(pm_hall* hp, double* pr, double* pp, double* vx, double* vy, double* vz) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     const int par = h->parity;
     pm_status s;
     if ((s = h->get(h->p[par], pr, h->nodes())) != PM_OK) return s;
@@ -599,7 +606,7 @@ pm_status pm_hall_set_tile(pm_hall* hp, int planes, int stages) {
 
 pm_status pm_hall_tile(pm_hall* hp, int* planes, int* stages) {
     Hall* h = reinterpret_cast<Hall*>(hp);
-    HALL_GUARD(h);
+    HALL_LOOK(h);
     if (planes) *planes = h->tma ? kHallTmaShapes[h->tshape].planes : 0;
     if (stages) *stages = h->tma ? kHallTmaShapes[h->tshape].stages : 0;
     return PM_OK;

@@ -115,6 +115,7 @@ struct Heat : Handle {
     // solid.rs:588-784 for a one-phase block; a block with void or a source is a filled one.
     void resolve() {
         uniform = mats.size() == 1 && vd.empty() && source.empty();
+        rate_is_known = false;
         gaps.clear();
         const size_t N = n();
         if (uniform) {
@@ -302,8 +303,16 @@ struct Heat : Handle {
         return total;
     }
 
-    // solid.rs:1148-1185
+    // solid.rs:1148-1185 where it does not follow the state, formed once per change of the block (resolve):
+    // a filled block's walks all its face cells.
+    mutable double rate_known = 0.0;
+    mutable bool rate_is_known = false;
     double worst_rate_now() const {
+        if (!rate_is_known) rate_known = form_worst_rate();
+        rate_is_known = true;
+        return rate_known;
+    }
+    double form_worst_rate() const {
         if (films.exposed == 0 || std::isnan(worst_rate)) return worst_rate;
         double worst = worst_rate;
         auto visit = [&](int i, int j, int k) {
@@ -622,6 +631,7 @@ struct Heat : Handle {
         const double joules = pending;
         if (joules == 0.0) return PM_OK;
         pending = 0.0;
+        mirror = false;
         const double rise = joules / cap_sum;  // solid.rs:1755
         PM_CUDA(launch_heat_rise(precision == PM_PLAIN_F64 ? field[parity].as<double>() : nullptr,
                                  precision == PM_PLAIN_F64 ? nullptr : field[parity].as<float>(), rise, n(),
@@ -659,10 +669,17 @@ struct Heat : Handle {
 
 using namespace pm;
 
-#define HEAT_GUARD(h)                                          \
+// Entry of a call that reads the handle or steps it (LOOK), and of every other (GUARD), which may
+// change the state block behind its mirror.
+#define HEAT_LOOK(h)                                          \
     do {                                                       \
         if (!(h)) return fail(PM_BAD_ARG, "null pm_heat");      \
         cudaSetDevice((h)->device);                            \
+    } while (0)
+#define HEAT_GUARD(h) \
+    do {               \
+        HEAT_LOOK(h);  \
+        (h)->mirror = false; \
     } while (0)
 
 extern "C" {
@@ -818,7 +835,7 @@ pm_status pm_heat_upload(pm_heat* hp, const double* kelvin, size_t n) {
 
 pm_status pm_heat_download(pm_heat* hp, double* kelvin, size_t n) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     if (!kelvin || n != h->n()) return fail(PM_BAD_ARG, "download: one value per cell");
     if (h->precision == PM_PLAIN_F64) {
         PM_CUDA(cudaMemcpyAsync(kelvin, h->field[h->parity].p, n * 8, cudaMemcpyDeviceToHost, h->stream()));
@@ -833,7 +850,7 @@ pm_status pm_heat_download(pm_heat* hp, double* kelvin, size_t n) {
 
 pm_status pm_heat_sample(pm_heat* hp, const double* lo, const double* hi, const int* samples, double* out, size_t n) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     SampleGrid g{};
     pm_status s = sample_grid_of(lo, hi, samples, out, n, g);
     if (s != PM_OK) return s;
@@ -849,13 +866,13 @@ pm_status pm_heat_sample(pm_heat* hp, const double* lo, const double* hi, const 
 
 pm_status pm_heat_max_stable_dt(pm_heat* hp, double* seconds) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     if (!seconds) return fail(PM_BAD_ARG, "null output");
     double rate;
     if (h->state_dependent()) {
         if (h->precision != PM_PLAIN_F64 && !h->radiating_f32())
             return fail(PM_UNSUPPORTED, "radiative gaps, and radiating films on blocks of several materials, are on the plain f64 form only");
-        pm_status s = h->read_state();  // the rate the last step (or the last change of state) left
+        pm_status s = h->latest_state();  // the rate the last step (or the last change of state) left
         if (s != PM_OK) return s;
         rate = h->host_state->rate_now;
     } else {
@@ -867,14 +884,14 @@ pm_status pm_heat_max_stable_dt(pm_heat* hp, double* seconds) {
 
 pm_status pm_heat_set_tolerance(pm_heat* hp, double tol) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     h->tolerance = tol;
     return PM_OK;
 }
 
 pm_status pm_heat_step(pm_heat* hp, double dt, long long nsteps, pm_violation* out) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     if (nsteps < 0) return fail(PM_BAD_ARG, "nsteps must be >= 0");
     if (nsteps == 0) return PM_OK;
     double rate;
@@ -883,7 +900,7 @@ pm_status pm_heat_step(pm_heat* hp, double dt, long long nsteps, pm_violation* o
         // state's rate, every later one on the device against the rate its own state gives
         if (h->precision != PM_PLAIN_F64 && !h->radiating_f32())
             return fail(PM_UNSUPPORTED, "radiative gaps, and radiating films on blocks of several materials, are on the plain f64 form only");
-        pm_status rs = h->read_state();
+        pm_status rs = h->latest_state();
         if (rs != PM_OK) return rs;
         rate = h->host_state->rate_now;
     } else {
@@ -932,9 +949,9 @@ pm_status pm_heat_step(pm_heat* hp, double dt, long long nsteps, pm_violation* o
 
 pm_status pm_heat_ledger(pm_heat* hp, pm_ledger* out) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     if (!out) return fail(PM_BAD_ARG, "null output");
-    pm_status s = h->read_state();
+    pm_status s = h->latest_state();
     if (s != PM_OK) return s;
     std::memset(out, 0, sizeof(*out));
     out->total = h->host_state->total;
@@ -983,7 +1000,7 @@ pm_status pm_heat_restore(pm_heat* hp) {
 
 pm_status pm_heat_step_kernel(pm_heat* hp, long long nsteps, char* name, int cap, long long* launches) {
     Heat* h = reinterpret_cast<Heat*>(hp);
-    HEAT_GUARD(h);
+    HEAT_LOOK(h);
     if (!name || cap < 1) return fail(PM_BAD_ARG, "step_kernel: a name buffer of one byte or more");
     const bool plain = h->precision == PM_PLAIN_F64;
     const bool filled = !h->uniform;

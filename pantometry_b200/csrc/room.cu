@@ -110,10 +110,17 @@ struct Room : Handle {
 
 using namespace pm;
 
-#define ROOM_GUARD(r)                                          \
+// Entry of a call that reads the handle or steps it (LOOK), and of every other (GUARD), which may
+// change the state block behind its mirror.
+#define ROOM_LOOK(r)                                          \
     do {                                                       \
         if (!(r)) return fail(PM_BAD_ARG, "null pm_room");      \
         cudaSetDevice((r)->device);                            \
+    } while (0)
+#define ROOM_GUARD(r) \
+    do {               \
+        ROOM_LOOK(r);  \
+        (r)->mirror = false; \
     } while (0)
 
 extern "C" {
@@ -153,7 +160,7 @@ pm_status pm_room_create(const pm_room_desc* d, pm_room** out) {
 
 pm_status pm_room_cells(pm_room* rp, int* nx, int* ny, double* dx) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     if (nx) *nx = r->nx;
     if (ny) *ny = r->ny;
     if (dx) *dx = r->dx;
@@ -190,7 +197,7 @@ pm_status pm_room_release(pm_room* rp, const double* pressure, size_t n) {
 
 pm_status pm_room_max_stable_dt(pm_room* rp, double* seconds) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     if (!seconds) return fail(PM_BAD_ARG, "null output");
     *seconds = r->speed <= 0.0 ? std::numeric_limits<double>::infinity() : r->dx / (r->speed * std::sqrt(2.0));
     return PM_OK;
@@ -198,14 +205,14 @@ pm_status pm_room_max_stable_dt(pm_room* rp, double* seconds) {
 
 pm_status pm_room_set_tolerance(pm_room* rp, double tol) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     r->tolerance = tol;
     return PM_OK;
 }
 
 pm_status pm_room_step(pm_room* rp, double dt, long long nsteps, pm_violation* out) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     if (nsteps < 0) return fail(PM_BAD_ARG, "nsteps must be >= 0");
     if (nsteps == 0) return PM_OK;
     // room.rs:369-380 (Room::courant, room.rs:336-338)
@@ -234,9 +241,9 @@ pm_status pm_room_step(pm_room* rp, double dt, long long nsteps, pm_violation* o
 
 pm_status pm_room_ledger(pm_room* rp, pm_ledger* out) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     if (!out) return fail(PM_BAD_ARG, "null output");
-    pm_status s = r->read_state();
+    pm_status s = r->latest_state();
     if (s != PM_OK) return s;
     std::memset(out, 0, sizeof(*out));
     const DevState* st = r->host_state;
@@ -252,7 +259,7 @@ pm_status pm_room_ledger(pm_room* rp, pm_ledger* out) {
 
 pm_status pm_room_download(pm_room* rp, double* pr, double* pp, double* vx, double* vy) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     const int par = r->parity;
     pm_status s;
     if ((s = r->get(r->p[par], pr, r->nodes())) != PM_OK) return s;
@@ -263,7 +270,7 @@ pm_status pm_room_download(pm_room* rp, double* pr, double* pp, double* vx, doub
 
 pm_status pm_room_sample(pm_room* rp, const double* lo, const double* hi, const int* samples, double* out, size_t n) {
     Room* r = reinterpret_cast<Room*>(rp);
-    ROOM_GUARD(r);
+    ROOM_LOOK(r);
     SampleGrid g{};
     pm_status s = sample_grid_of(lo, hi, samples, out, n, g);
     if (s != PM_OK) return s;

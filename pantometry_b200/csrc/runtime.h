@@ -75,6 +75,12 @@ struct Handle {
     DBuf partials;   // per-block partial sums
     DBuf sampled;    // the samples of the last pm_*_sample call
     DevState* host_state = nullptr;  // pinned mirror
+    // host_state holds the device's state block as the last step call read it, and nothing has been done
+    // to the handle since: the next call then neither reads it again nor, where nothing in it is to
+    // change, writes it. A frame of a small scene (one step, a ledger) made three synchronising copies
+    // without it, about 40 of its 60 µs. Every entry point that may launch work or change the block
+    // clears it (its guard); only the end of a step call that ran through sets it.
+    bool mirror = false;
     double tolerance = -1.0;         // no audit: plain `Domain::step`; set one to audit every step
     std::string refusal_site;        // where a step refused on the device (kRefused) is reported
     unsigned resident = 148 * kBlocksPerSM;  // upper bound of any persistent grid (partials sizing)
@@ -105,8 +111,9 @@ struct Handle {
         return e;
     }
     pm_status read_state();                    // device → host_state, synchronising
+    pm_status latest_state() { return mirror ? PM_OK : read_state(); }
     pm_status write_state();                   // host_state → device
-    pm_status begin_call();                    // clear the previous call's violation
+    pm_status begin_call();                    // clear the previous call's violation; host_state is current
     // Run `n` steps with `one(parity)` launching a single step from buffer `parity`.
     // `pingpong`: each step flips the parity.
     template <typename F>

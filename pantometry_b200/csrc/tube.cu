@@ -114,10 +114,17 @@ struct Tube : Handle {
 
 using namespace pm;
 
-#define TUBE_GUARD(t)                                          \
+// Entry of a call that reads the handle or steps it (LOOK), and of every other (GUARD), which may
+// change the state block behind its mirror.
+#define TUBE_LOOK(t)                                          \
     do {                                                       \
         if (!(t)) return fail(PM_BAD_ARG, "null pm_tube");      \
         cudaSetDevice((t)->device);                            \
+    } while (0)
+#define TUBE_GUARD(t) \
+    do {               \
+        TUBE_LOOK(t);  \
+        (t)->mirror = false; \
     } while (0)
 
 extern "C" {
@@ -154,7 +161,7 @@ pm_status pm_tube_create(const pm_tube_desc* d, pm_tube** out) {
 
 pm_status pm_tube_cells(pm_tube* tp, int* n, double* dx) {
     Tube* t = reinterpret_cast<Tube*>(tp);
-    TUBE_GUARD(t);
+    TUBE_LOOK(t);
     if (n) *n = t->n;
     if (dx) *dx = t->dx;
     return PM_OK;
@@ -197,7 +204,7 @@ pm_status pm_tube_release(pm_tube* tp, const double* pressure, size_t n) {
 
 pm_status pm_tube_max_stable_dt(pm_tube* tp, double* seconds) {
     Tube* t = reinterpret_cast<Tube*>(tp);
-    TUBE_GUARD(t);
+    TUBE_LOOK(t);
     if (!seconds) return fail(PM_BAD_ARG, "null output");
     const double inf = std::numeric_limits<double>::infinity();
     if (t->speed <= 0.0) { *seconds = inf; return PM_OK; }
@@ -216,14 +223,14 @@ pm_status pm_tube_max_stable_dt(pm_tube* tp, double* seconds) {
 
 pm_status pm_tube_set_tolerance(pm_tube* tp, double tol) {
     Tube* t = reinterpret_cast<Tube*>(tp);
-    TUBE_GUARD(t);
+    TUBE_LOOK(t);
     t->tolerance = tol;
     return PM_OK;
 }
 
 pm_status pm_tube_step(pm_tube* tp, double dt, long long nsteps, pm_violation* out) {
     Tube* t = reinterpret_cast<Tube*>(tp);
-    TUBE_GUARD(t);
+    TUBE_LOOK(t);
     if (nsteps < 0) return fail(PM_BAD_ARG, "nsteps must be >= 0");
     if (nsteps == 0) return PM_OK;
     // lib.rs:517-527 (Tube::courant, lib.rs:358-360)
@@ -252,9 +259,9 @@ pm_status pm_tube_step(pm_tube* tp, double dt, long long nsteps, pm_violation* o
 
 pm_status pm_tube_ledger(pm_tube* tp, pm_ledger* out) {
     Tube* t = reinterpret_cast<Tube*>(tp);
-    TUBE_GUARD(t);
+    TUBE_LOOK(t);
     if (!out) return fail(PM_BAD_ARG, "null output");
-    pm_status s = t->read_state();
+    pm_status s = t->latest_state();
     if (s != PM_OK) return s;
     std::memset(out, 0, sizeof(*out));
     const DevState* st = t->host_state;
@@ -270,7 +277,7 @@ pm_status pm_tube_ledger(pm_tube* tp, pm_ledger* out) {
 
 pm_status pm_tube_download(pm_tube* tp, double* pr, double* pp, double* v) {
     Tube* t = reinterpret_cast<Tube*>(tp);
-    TUBE_GUARD(t);
+    TUBE_LOOK(t);
     const int par = t->parity;
     pm_status s;
     if ((s = t->get(t->p[par], pr, (size_t)t->n)) != PM_OK) return s;
