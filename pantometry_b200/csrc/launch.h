@@ -176,6 +176,11 @@ template <typename Real> cudaError_t launch_ens(const EnsArgs<Real>& a, bool mea
 
 // Element-wise conversions between the caller's f64 arrays and an f32 store.
 template <typename Real> cudaError_t launch_room(const RoomArgs<Real>& a, cudaStream_t s);
+// Many steps of a room in one launch of one cluster of `blocks` thread blocks (room_steps).
+template <typename Real> cudaError_t launch_room_steps(const RoomStepsArgs<Real>& a, int blocks, cudaStream_t s);
+// The largest cluster (at most kRoomMaxCluster blocks, at most a block per row) that holds an nx × ny
+// room in shared memory on the current device, 0 where none does; *rows: the most rows of a block.
+template <typename Real> int room_steps_cluster(int nx, int ny, int* rows);
 template <typename Real> cudaError_t launch_room_measure(const RoomMeasureArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_tube(const TubeArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_bar(const BarArgs<Real>& a, cudaStream_t s);

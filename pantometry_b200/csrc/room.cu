@@ -48,6 +48,32 @@ struct Room : Handle {
         a.partials = partials.as<double>();
         return a;
     }
+    // Steps of a call in one launch of one cluster (room_steps), where the room fits one.
+    int cluster = -1, cluster_rows = 0;  // −1: not asked yet; 0: it does not
+    int steps_cluster() {
+        if (cluster < 0)
+            cluster = precision == PM_PLAIN_F64 ? room_steps_cluster<double>(nx, ny, &cluster_rows)
+                                                : room_steps_cluster<float>(nx, ny, &cluster_rows);
+        return cluster;
+    }
+    template <typename Real>
+    pm_status run_cluster(long long n, double h) {
+        const RoomArgs<Real> one = args<Real>(parity, h, false);
+        RoomStepsArgs<Real> a{};
+        a.nx = nx; a.ny = ny; a.rows = cluster_rows;
+        a.gain = one.gain; a.scale = one.scale; a.knode = one.knode; a.kface = one.kface;
+        a.st = one.st;
+        while (n > 0) {
+            a.nsteps = (int)std::min<long long>(n, kRoomChunk);
+            for (int q = 0; q < 2; ++q) {
+                a.p[q] = p[parity ^ q].as<Real>(); a.vx[q] = vx[parity ^ q].as<Real>(); a.vy[q] = vy[parity ^ q].as<Real>();
+            }
+            PM_CUDA(launch_room_steps<Real>(a, cluster, stream()));
+            parity ^= a.nsteps & 1;
+            n -= a.nsteps;
+        }
+        return PM_OK;
+    }
     cudaError_t launch(int par, double h, bool starting, cudaStream_t s) const {
         if (precision == PM_PLAIN_F64) return launch_room<double>(args<double>(par, h, starting), s);
         return launch_room<float>(args<float>(par, h, starting), s);
@@ -233,7 +259,10 @@ pm_status pm_room_step(pm_room* rp, double dt, long long nsteps, pm_violation* o
         r->staggered = true;
         remaining -= 1;
     }
-    s = r->run_steps(remaining, dt, true, [r, dt](int par, cudaStream_t st) { return r->launch(par, dt, false, st); });
+    if (remaining >= 2 && r->steps_cluster() > 0)
+        s = r->precision == PM_PLAIN_F64 ? r->run_cluster<double>(remaining, dt) : r->run_cluster<float>(remaining, dt);
+    else
+        s = r->run_steps(remaining, dt, true, [r, dt](int par, cudaStream_t st) { return r->launch(par, dt, false, st); });
     if (s != PM_OK) return s;
     return r->finish_call(before, out, r->name + " (its own books, against what it moved on the bus)",
                           r->name + " (starting the leapfrog)", true);

@@ -15,6 +15,8 @@
 // room_measure — the invariant of a state, for the datum of a release and for a restore.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace pm {
@@ -90,6 +92,165 @@ static __global__ void __launch_bounds__(256) room_step(RoomArgs<Real> a) {
         st->invariant = invariant;
         audit_and_commit(st, total, scale_l);
     });
+}
+
+// Many steps of a room in one launch, the room held on the chip: one thread-block cluster, its blocks
+// taking the rows between them, each block's rows of p, vx and vy in its shared memory. A step reads
+// the old state and writes the new one in shared memory; a block also writes its first and last rows'
+// new pressure into its neighbours' halo rows (distributed shared memory), and keeps its own copy of the
+// vy faces below its first row, formed by the expression the block below forms them with. One cluster
+// barrier ends the step. A room is a few thousand nodes, so a launch a step spent its time on the launch,
+// the first loads and the books' round trips: 4.56 µs a step at 101 × 72 nodes in f64, 1.43 here; 41 × 30 in
+// FP32 4.58 and 1.20. Rooms past a cluster's shared memory (about 270 × 190 nodes in f64) and single steps
+// keep room_step.
+//
+// The books stay off that path, as in the many-step heat kernels: each warp leaves its sum of step s in
+// block 0, whose last warp (it takes no nodes) reduces and audits it while the others run step s + 1. A
+// failed audit is told to every block before step s + 1's barrier, and the call ends with step s's
+// state: p holds three steps, so s and s − 1 are intact, and vx and vy two.
+constexpr int kRoomThreads = 512;  // nodes are taken by these; one warp more keeps the books
+constexpr int kRoomMaxCluster = 16;
+constexpr int kRoomChunk = 4096;  // steps a launch
+
+template <typename Real>
+struct RoomStepsArgs {
+    Real* p[2];  // by parity; the call starts from p[0], vx[0], vy[0]
+    Real* vx[2];
+    Real* vy[2];
+    int nx, ny;
+    int rows;    // the most rows a block holds
+    int nsteps;
+    Real gain, scale;
+    double knode, kface;
+    DevState* st;
+};
+template <typename Real>
+inline size_t room_steps_smem(int nx, int rows) {
+    return sizeof(Real) * (size_t)nx * (3 * (size_t)(rows + 2) + 2 * (size_t)rows + 2 * (size_t)(rows + 1));
+}
+
+template <typename Real>
+static __global__ void __launch_bounds__(kRoomThreads + 32, 1) room_steps(RoomStepsArgs<Real> a) {
+    namespace cg = cooperative_groups;
+    constexpr int WARPS = kRoomThreads / 32;
+    extern __shared__ __align__(16) unsigned char room_smem[];
+    __shared__ double part[2][kRoomMaxCluster * WARPS];  // block 0's: each warp's sum of a step, by its parity
+    __shared__ DevState books;                           // block 0's
+    __shared__ int stop;
+    if (a.st->violated) return;  // every block reads the same word
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
+    const int nx = a.nx, ny = a.ny, rows = a.rows;
+    const int r0 = (int)((long long)ny * rank / blocks), r1 = (int)((long long)ny * (rank + 1) / blocks);
+    Real* const P = reinterpret_cast<Real*>(room_smem);  // [3][rows + 2][nx]: rows r0 − 1 .. r1
+    Real* const VX = P + (size_t)3 * (rows + 2) * nx;     // [2][rows][nx]: rows r0 .. r1 − 1
+    Real* const VY = VX + (size_t)2 * rows * nx;          // [2][rows + 1][nx]: faces above rows r0 − 1 .. r1 − 1
+    const size_t pslot = (size_t)(rows + 2) * nx, xslot = (size_t)rows * nx, yslot = (size_t)(rows + 1) * nx;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool keeper = rank == 0 && warp == WARPS;
+    for (int l = tid; l < (r1 - r0 + 2) * nx; l += kRoomThreads + 32) {
+        const int i = l % nx, j = r0 - 1 + l / nx;
+        if (j >= 0 && j < ny) P[l] = a.p[0][i + (size_t)nx * j];
+        if (j >= 0 && j < ny - 1 && j < r1) VY[l] = a.vy[0][i + (size_t)nx * j];
+        if (j >= r0 && j < r1 && i < nx - 1) VX[l - nx] = a.vx[0][i + (size_t)(nx - 1) * j];
+    }
+    if (tid == 0) stop = 0;
+    if (keeper && lane == 0) books = *a.st;
+    Real* const below_p = rank > 0 ? cluster.map_shared_rank(P, rank - 1) : nullptr;
+    Real* const above_p = rank + 1 < blocks ? cluster.map_shared_rank(P, rank + 1) : nullptr;
+    const int below_rows = rank > 0 ? r0 - (int)((long long)ny * (rank - 1) / blocks) : 0;
+    double* const sums = cluster.map_shared_rank(&part[0][0], 0) + rank * WARPS;
+    cluster.sync();
+
+    auto audit = [&](int s) {  // the keeper: step s's sums into the books
+        double v[1] = {0.0};
+        for (int w = lane; w < blocks * WARPS; w += 32) v[0] += part[s & 1][w];
+        warp_sum<1>(v);
+        int failed = 0;
+        if (lane == 0) {
+            const double invariant = v[0];
+            double total = 0.0, scale = 0.0;
+            ledger_add(total, scale, invariant + books.offset);  // room.rs:480-482
+            books.part[0] = total;
+            books.invariant = invariant;
+            audit_and_commit(&books, total, scale);
+            failed = books.violated;
+        }
+        return __shfl_sync(0xffffffffu, failed, 0) != 0;
+    };
+
+    const Real gain = a.gain, scale = a.scale;
+    const int mine = (r1 - r0) * nx;
+    int done = a.nsteps, slot = 0;  // p's slot of the present state
+    bool failed = false;
+    for (int s = 0; s < a.nsteps; ++s) {
+        const int next = slot == 2 ? 0 : slot + 1;
+        if (warp < WARPS) {
+            const Real* p0 = P + slot * pslot + nx;  // row r0
+            const Real* x0 = VX + (s & 1) * xslot;
+            const Real* y0 = VY + (s & 1) * yslot + nx;  // the faces above row r0
+            Real* p1 = P + next * pslot + nx;
+            Real* x1 = VX + ((s + 1) & 1) * xslot;
+            Real* y1 = VY + ((s + 1) & 1) * yslot + nx;
+            double acc[1] = {0.0};
+            int i = tid % nx, l = tid / nx;
+            for (int c = tid; c < mine; c += kRoomThreads) {
+                const int j = r0 + l;
+                const Real pc = p0[c];
+                // room_step's expressions
+                const Real left = i > 0 ? x0[c - 1] - gain * (pc - p0[c - 1]) : Real(0);
+                const Real right = i < nx - 1 ? x0[c] - gain * (p0[c + 1] - pc) : Real(0);
+                const Real below = j > 0 ? y0[c - nx] - gain * (pc - p0[c - nx]) : Real(0);
+                const Real above = j < ny - 1 ? y0[c] - gain * (p0[c + nx] - pc) : Real(0);
+                x1[c] = right;
+                y1[c] = above;
+                if (l == 0) y1[c - nx] = below;
+                const Real wi = (i == 0 || i == nx - 1) ? Real(2) : Real(1);
+                const Real wj = (j == 0 || j == ny - 1) ? Real(2) : Real(1);
+                const Real np = pc - scale * (wi * (right - left) + wj * (above - below));
+                p1[c] = np;
+                if (l == 0 && below_p) below_p[next * pslot + (size_t)(below_rows + 1) * nx + i] = np;
+                if (j == r1 - 1 && above_p) above_p[next * pslot + i] = np;
+                const double si = room_share(i, nx), sj = room_share(j, ny);
+                const double dr = (double)right, da = (double)above;
+                acc[0] += (si * sj) * a.knode * (double)np * (double)pc + sj * a.kface * (dr * dr) + si * a.kface * (da * da);
+                i += kRoomThreads % nx;
+                l += kRoomThreads / nx;
+                if (i >= nx) {
+                    i -= nx;
+                    ++l;
+                }
+            }
+            warp_sum<1>(acc);
+            if (lane == 0) sums[(s & 1) * (kRoomMaxCluster * WARPS) + warp] = acc[0];
+        } else if (keeper && s > 0 && audit(s - 1)) {
+            if (lane < blocks) *cluster.map_shared_rank(&stop, lane) = 1;
+        }
+        cluster.sync();
+        if (stop) {  // step s − 1 failed its audit: the state it left is the present slot's
+            failed = true;
+            done = s;
+            break;
+        }
+        slot = next;
+    }
+    if (keeper) {
+        if (!failed) audit(a.nsteps - 1);
+        if (lane == 0) {
+            books.counter = 0u;
+            *a.st = books;
+        }
+    }
+    // the state after `done` steps (at least one), p's before it as the previous pressure
+    const int par = done & 1, before = slot == 0 ? 2 : slot - 1;
+    for (int c = tid; c < mine; c += kRoomThreads + 32) {
+        const int i = c % nx, j = r0 + c / nx;
+        const size_t g = i + (size_t)nx * j;
+        a.p[par][g] = P[slot * pslot + nx + c];
+        a.p[par ^ 1][g] = P[before * pslot + nx + c];
+        if (i < nx - 1) a.vx[par][i + (size_t)(nx - 1) * j] = VX[par * xslot + c];
+        if (j < ny - 1) a.vy[par][g] = VY[par * yslot + nx + c];
+    }
 }
 
 template <typename Real>
