@@ -38,7 +38,8 @@ struct Cavity : Handle {
     double mu_one = 0.0;
     std::vector<uint8_t> solid;
     bool any_solid = false;
-    DBuf dsolid;
+    DBuf dsolid;  // the solid cells
+    DBuf dedges;  // the edges that touch one, by lattice node (solid_edges)
     // fields: ping-pong pairs, f[parity] holds the state
     DBuf f[2][6];  // ex ey ez hx hy hz
     DBuf keep[3];
@@ -210,42 +211,6 @@ struct Cavity : Handle {
     }
 
     template <typename Real>
-    YeeEArgs<Real> eargs(double dt) const {
-        YeeEArgs<Real> a{};
-        const DBuf* c = f[parity];
-        a.ex = c[0].as<Real>(); a.ey = c[1].as<Real>(); a.ez = c[2].as<Real>();
-        a.hx = c[3].as<Real>(); a.hy = c[4].as<Real>(); a.hz = c[5].as<Real>();
-        a.nx = nx; a.ny = ny; a.nz = nz;
-        a.dt = dt; a.dx = dx; a.volume = volume();
-        a.uniform = uniform ? 1 : 0;
-        // cavity.rs:1391-1397 at the uniform edge ε and σ
-        const double half = sig_u * dt / (2.0 * eps_u);
-        for (int q = 0; q < 3; ++q) {
-            a.decay[q] = (Real)((1.0 - half) / (1.0 + half));
-            a.gain[q] = (Real)((dt / (eps_u * dx)) / (1.0 + half));
-            a.sigma_u[q] = sig_u;
-        }
-        a.eps0 = deps[0].as<double>(); a.eps1 = deps[1].as<double>(); a.eps2 = deps[2].as<double>();
-        a.sig0 = dsig[0].as<double>(); a.sig1 = dsig[1].as<double>(); a.sig2 = dsig[2].as<double>();
-        a.solid = any_solid ? dsolid.as<uint8_t>() : nullptr;
-        a.src = src;
-        a.current = current.as<double>();
-        a.ncurrent = ncurrent;
-        a.with_source = src >= 0 ? 1 : 0;
-        if (src >= 0) {
-            a.eps_src = uniform ? eps_u : eps[2][(size_t)src];
-            a.sig_src = uniform ? sig_u : sig[2][(size_t)src];
-        }
-        const unsigned w = wave_of(sizeof(Real) == 8 ? kYeeEF64 : kYeeEF32);
-        a.tiles = make_tiles(nx + 1, ny + 1, nz + 1, choose_zc(nx + 1, ny + 1, nz + 1, w));
-        a.nblocks = grid_for(a.tiles, w);
-        a.st = state.as<DevState>();
-        a.partials = partials.as<double>();
-        return a;
-    }
-
-    // The fused step from buffer set `par` into `par ^ 1`.
-    template <typename Real>
     YeeStepArgs<Real> sargs(int par, double dt) const {
         YeeStepArgs<Real> a{};
         for (int q = 0; q < 6; ++q) {
@@ -284,7 +249,7 @@ struct Cavity : Handle {
             a.mu_var = mu_var ? 1 : 0;
             if (!mu_var) { a.mu_u = mu_one; a.ch = (Real)(a.g / mu_one); }
         }
-        a.solid = any_solid ? dsolid.as<uint8_t>() : nullptr;
+        a.solid = any_solid ? dedges.as<uint8_t>() : nullptr;
         a.src_i = a.src_j = a.src_k = -1;
         if (src >= 0) {
             a.src_i = (int)(src % (nx + 1));
@@ -390,6 +355,24 @@ struct Cavity : Handle {
         for (int q = 0; q < 6; ++q)  // the other set back to a zero-padded lattice
             PM_CUDA(cudaMemsetAsync(f[home ^ 1][q].p, 0, lattice() * 4, stream()));
         PM_CUDA(cudaStreamSynchronize(stream()));
+        return PM_OK;
+    }
+
+    // cavity.rs:304-331: the twelve edges of every solid cell, as the step kernels read them.
+    pm_status upload_edges() {
+        const size_t sy = (size_t)nx + 1, sz = sy * ((size_t)ny + 1);
+        std::vector<uint8_t> e(sz * ((size_t)nz + 1), 0);
+        for (int k = 0; k < nz; ++k)
+            for (int j = 0; j < ny; ++j)
+                for (int i = 0; i < nx; ++i) {
+                    if (!solid[i + (size_t)nx * (j + (size_t)ny * k)]) continue;
+                    uint8_t* n = &e[i + sy * j + sz * k];
+                    for (size_t q : {size_t(0), sy, sz, sy + sz}) n[q] |= 1;
+                    for (size_t q : {size_t(0), size_t(1), sz, 1 + sz}) n[q] |= 2;
+                    for (size_t q : {size_t(0), size_t(1), sy, 1 + sy}) n[q] |= 4;
+                }
+        PM_CUDA(dedges.alloc(e.size()));
+        PM_CUDA(put_sync(dedges.p, e.data(), e.size()));
         return PM_OK;
     }
 
@@ -890,6 +873,7 @@ pm_status pm_cavity_obstruct(pm_cavity* cp, const uint8_t* mask, size_t n) {
     if (hs != PM_OK) return hs;
     PM_CUDA(c->dsolid.alloc(c->cells()));
     PM_CUDA(c->put_sync(c->dsolid.p, c->solid.data(), c->cells()));
+    if (pm_status es = c->upload_edges(); es != PM_OK) return es;
     c->drop_graphs();
     // cavity.rs:293 `enforce_solid` now, on the host copy of E
     std::vector<double> e[3];

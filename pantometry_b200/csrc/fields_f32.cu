@@ -47,11 +47,6 @@ cudaError_t launch_yee_h<float>(const YeeHArgs<float>& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 template <>
-cudaError_t launch_yee_e<float>(const YeeEArgs<float>& a, cudaStream_t s) {
-    yee_e<float><<<a.nblocks, tile_block(), 0, s>>>(a);
-    return cudaGetLastError();
-}
-template <>
 cudaError_t launch_yee_step<float>(const YeeStepArgs<float>& a, cudaStream_t s) {
     const int smem = (int)yee_smem_bytes<float>();
     auto k = a.uniform ? (a.solid ? yee_step<float, true, true> : yee_step<float, true, false>)
@@ -331,7 +326,6 @@ int occupancy_f32(KernelId id) {
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, hall_step<float, false>, 256, hall_smem_bytes<float>());
             break;
         case kYeeHF32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, yee_h<float>, 256, 0); break;
-        case kYeeEF32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, yee_e<float>, 256, 0); break;
         case kYeeStepF32:
             e = allow_smem(yee_step<float, false, true>, (int)yee_smem_bytes<float>());
             if (e != cudaSuccess) break;

@@ -66,7 +66,7 @@ inline cudaError_t launch_smem(void (*kernel)(P...), dim3 grid, dim3 block, int 
 // Resident blocks per SM of each step kernel at 256 threads (cudaOccupancyMaxActiveBlocksPer-
 // Multiprocessor, asked once per kernel and device), so a persistent grid is exactly one full wave.
 enum KernelId : int {
-    kHeatPlain = 0, kHeatF32, kHallF64, kHallF32, kYeeHF64, kYeeHF32, kYeeEF64, kYeeEF32, kYeeStepF64, kYeeStepF32,
+    kHeatPlain = 0, kHeatF32, kHallF64, kHallF32, kYeeHF64, kYeeHF32, kYeeStepF64, kYeeStepF32,
     kEnsF64, kEnsF32, kHallTma, kYeeTma, kYeeTmaMedia, kEnsTma, kRoomF64, kRoomF32, kTubeF64, kTubeF32, kBarF64, kBarF32, kHeatF32Quad, kEnsF32Quad, kHeatPlainPair, kEnsF64Pair, kHeatPlainSteps, kHeatF32QuadSteps, kHeatPlainSteps32, kHeatF32QuadSteps32, kHeatTma,
     kHallTmaShape1, kHallTmaShape2, kHallTmaShape3,  // kHallTma is shape 0
     kYeeTmaShape1, kYeeTmaShape2, kYeeTmaMediaShape1,  // kYeeTma and kYeeTmaMedia are shape 0 of each form
@@ -114,7 +114,6 @@ cudaError_t launch_heat_rise(double* t64, float* d32, double rise, size_t n, con
 template <typename Real> cudaError_t launch_hall(const HallArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_hall_measure(const HallMeasureArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_yee_h(const YeeHArgs<Real>& a, cudaStream_t s);
-template <typename Real> cudaError_t launch_yee_e(const YeeEArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_yee_step(const YeeStepArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_yee_measure(const YeeHArgs<Real>& a, double* out2, cudaStream_t s);
 template <typename Real> cudaError_t launch_yee_walls(const YeeWallArgs<Real>& a, cudaStream_t s);

@@ -65,11 +65,6 @@ cudaError_t launch_yee_h<double>(const YeeHArgs<double>& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 template <>
-cudaError_t launch_yee_e<double>(const YeeEArgs<double>& a, cudaStream_t s) {
-    yee_e<double><<<a.nblocks, tile_block(), 0, s>>>(a);
-    return cudaGetLastError();
-}
-template <>
 cudaError_t launch_yee_step<double>(const YeeStepArgs<double>& a, cudaStream_t s) {
     const int smem = (int)yee_smem_bytes<double>();
     auto k = a.uniform ? (a.solid ? yee_step<double, true, true> : yee_step<double, true, false>)
@@ -245,7 +240,6 @@ int occupancy_f64(KernelId id) {
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, hall_step<double, false>, 256, hall_smem_bytes<double>());
             break;
         case kYeeHF64: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, yee_h<double>, 256, 0); break;
-        case kYeeEF64: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, yee_e<double>, 256, 0); break;
         case kYeeStepF64:
             e = allow_smem(yee_step<double, false, true>, (int)yee_smem_bytes<double>());
             if (e != cudaSuccess) break;

@@ -2,17 +2,14 @@
 //
 // Per step the reference runs: three H passes; a clone of H; the invariant — two full passes
 // that pair Eⁿ with H⁻ and H⁺ (cavity.rs:1490-1496); three E passes; the wall pass; the
-// obstacle pass. Here a step is two kernels over the (nx+1)(ny+1)(nz+1) node lattice:
+// obstacle pass. Here a step is one pass over the (nx+1)(ny+1)(nz+1) node lattice, yee_step (and
+// yee_tma_step, its TMA-staged FP32 form), described below. Beside it
 //
 //   yee_h  — H⁺ = H⁻ − (dt/dx)/μ · curl Eⁿ for every face (cavity.rs:1346-1379), in place
 //            (each face is read and written by its own thread only), with the invariant's two
 //            halves accumulated in the same pass: ½εEⁿ² over the edges that share the thread's
-//            lattice index (cavity.rs:776-847) and ½μ H⁺·H⁻ over its faces (cavity.rs:854-905).
-//            H⁻ is the value in the register before the store, so the clone disappears.
-//   yee_e  — Eⁿ⁺¹ on interior edges with the semi-implicit loss (cavity.rs:1383-1452), zero on
-//            conducting walls (cavity.rs:1239-1293), zero on edges touching a solid cell
-//            (cavity.rs:304-331); the Joule loss and the source work in FP64; then the ledger
-//            `invariant + dissipated` (cavity.rs:1520-1524) and the audit in the last block.
+//            lattice index (cavity.rs:776-847) and ½μ H⁺·H⁻ over its faces (cavity.rs:854-905):
+//            the half step that starts the leapfrog and the released mode's invariant.
 //
 // Real = double with --fmad=false is the plain form, bit-exact with `Cavity::step`.
 #pragma once
@@ -142,37 +139,6 @@ static __global__ void __launch_bounds__(256) yee_h(YeeHArgs<Real> a) {
 }
 
 template <typename Real>
-struct YeeEArgs {
-    Real* __restrict__ ex;
-    Real* __restrict__ ey;
-    Real* __restrict__ ez;
-    const Real* __restrict__ hx;
-    const Real* __restrict__ hy;
-    const Real* __restrict__ hz;
-    int nx, ny, nz;
-    double dt, dx, volume;
-    int uniform;
-    Real decay[3], gain[3];             // uniform: per component, from the edge-mean ε and σ
-    double sigma_u[3];
-    const double* __restrict__ eps0;    // general: ε, σ per edge component
-    const double* __restrict__ eps1;
-    const double* __restrict__ eps2;
-    const double* __restrict__ sig0;
-    const double* __restrict__ sig1;
-    const double* __restrict__ sig2;
-    const uint8_t* __restrict__ solid;  // per cell, or null
-    long long src;                      // Ez edge with a soft current (extension), or -1
-    const double* __restrict__ current;
-    long long ncurrent;
-    double eps_src, sig_src;            // ε, σ at the source edge
-    int with_source;
-    Tiles tiles;
-    DevState* st;
-    double* partials;
-    unsigned nblocks;
-};
-
-template <typename Real>
 __device__ __forceinline__ void coefficients(double eps, double sigma, double dt, double dx, Real& decay, Real& gain) {
     // cavity.rs:1391-1397
     const double half = sigma * dt / (2.0 * eps);
@@ -180,120 +146,12 @@ __device__ __forceinline__ void coefficients(double eps, double sigma, double dt
     gain = (Real)((dt / (eps * dx)) / (1.0 + half));
 }
 
-__device__ __forceinline__ bool touches_solid(const uint8_t* solid, int nx, int ny, int nz, int ci0, int ci1,
-                                              int cj0, int cj1, int ck0, int ck1) {
-    for (int kk = ck0; kk <= ck1; ++kk)
-        for (int jj = cj0; jj <= cj1; ++jj)
-            for (int ii = ci0; ii <= ci1; ++ii)
-                if (ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz &&
-                    solid[(size_t)ii + (size_t)nx * ((size_t)jj + (size_t)ny * kk)])
-                    return true;
-    return false;
-}
-
-template <typename Real>
-static __global__ void __launch_bounds__(256) yee_e(YeeEArgs<Real> a) {
-    DevState* st = a.st;
-    if (st->violated) return;
-    const int nx = a.nx, ny = a.ny, nz = a.nz;
-    const size_t sEx = (size_t)nx * (ny + 1), sEy = (size_t)(nx + 1) * ny, sEz = (size_t)(nx + 1) * (ny + 1);
-    const size_t sHx = (size_t)(nx + 1) * ny, sHy = (size_t)nx * (ny + 1), sHz = (size_t)nx * ny;
-    const long long step = st->steps;
-    const double jsrc = (a.with_source && step < a.ncurrent) ? a.current[step] : 0.0;
-    const double dt = a.dt;
-    double acc[2] = {0.0, 0.0};  // Joule loss, source work
-    for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x) {
-        const int tx = (int)(t % a.tiles.ntx);
-        const long long r = t / a.tiles.ntx;
-        const int i = tx * 32 + threadIdx.x;
-        const int j = (int)(r % a.tiles.nty) * 8 + threadIdx.y;
-        const int k0 = (int)(r / a.tiles.nty) * a.tiles.zc;
-        const int k1 = min(nz + 1, k0 + a.tiles.zc);
-        if (i > nx || j > ny) continue;
-        const size_t ex0 = (size_t)i + (size_t)nx * j, ey0 = (size_t)i + (size_t)(nx + 1) * j;
-        const size_t ez0 = (size_t)i + (size_t)(nx + 1) * j;
-        const size_t hx0 = (size_t)i + (size_t)(nx + 1) * j, hy0 = (size_t)i + (size_t)nx * j, hz0 = (size_t)i + (size_t)nx * j;
-        // hy(i, j, k-1) and hx(i, j, k-1), carried from the previous plane
-        const bool xin = i >= 1 && i < nx, yin = j >= 1 && j < ny;
-        Real hy_km = (k0 >= 1 && i < nx && k0 - 1 < nz) ? a.hy[hy0 + sHy * (k0 - 1)] : Real(0);
-        Real hx_km = (k0 >= 1 && j < ny && k0 - 1 < nz) ? a.hx[hx0 + sHx * (k0 - 1)] : Real(0);
-        for (int k = k0; k < k1; ++k) {
-            const bool zin = k < nz, kint = k >= 1 && k < nz;
-            const Real hy_k = (i < nx && zin) ? a.hy[hy0 + sHy * k] : Real(0);
-            const Real hx_k = (j < ny && zin) ? a.hx[hx0 + sHx * k] : Real(0);
-            if (i < nx) {  // ex over nx × (ny+1) × (nz+1); interior j in 1..ny-1, k in 1..nz-1
-                const size_t idx = ex0 + sEx * k;
-                Real v = Real(0);
-                if (yin && kint) {
-                    const Real curl = (a.hz[hz0 + sHz * k] - a.hz[hz0 - nx + sHz * k]) - (hy_k - hy_km);
-                    Real decay = a.decay[0], gain = a.gain[0];
-                    double s = a.sigma_u[0];
-                    if (!a.uniform) { s = a.sig0[idx]; coefficients<Real>(a.eps0[idx], s, dt, a.dx, decay, gain); }
-                    const Real before = a.ex[idx];
-                    v = decay * before + gain * curl;
-                    const double mid = 0.5 * ((double)before + (double)v);
-                    acc[0] += s * mid * mid * dt * a.volume;
-                }
-                if (a.solid && touches_solid(a.solid, nx, ny, nz, i, i, j - 1, j, k - 1, k)) v = Real(0);
-                a.ex[idx] = v;
-            }
-            if (j < ny) {  // ey over (nx+1) × ny × (nz+1); interior i in 1..nx-1, k in 1..nz-1
-                const size_t idx = ey0 + sEy * k;
-                Real v = Real(0);
-                if (xin && kint) {
-                    const Real curl = (hx_k - hx_km) - (a.hz[hz0 + sHz * k] - a.hz[hz0 - 1 + sHz * k]);
-                    Real decay = a.decay[1], gain = a.gain[1];
-                    double s = a.sigma_u[1];
-                    if (!a.uniform) { s = a.sig1[idx]; coefficients<Real>(a.eps1[idx], s, dt, a.dx, decay, gain); }
-                    const Real before = a.ey[idx];
-                    v = decay * before + gain * curl;
-                    const double mid = 0.5 * ((double)before + (double)v);
-                    acc[0] += s * mid * mid * dt * a.volume;
-                }
-                if (a.solid && touches_solid(a.solid, nx, ny, nz, i - 1, i, j, j, k - 1, k)) v = Real(0);
-                a.ey[idx] = v;
-            }
-            if (zin) {  // ez over (nx+1) × (ny+1) × nz; interior i in 1..nx-1, j in 1..ny-1
-                const size_t idx = ez0 + sEz * k;
-                Real v = Real(0);
-                if (xin && yin) {
-                    const Real curl = (hy_k - a.hy[hy0 - 1 + sHy * k]) - (hx_k - a.hx[hx0 - (nx + 1) + sHx * k]);
-                    Real decay = a.decay[2], gain = a.gain[2];
-                    double s = a.sigma_u[2];
-                    if (!a.uniform) { s = a.sig2[idx]; coefficients<Real>(a.eps2[idx], s, dt, a.dx, decay, gain); }
-                    const Real before = a.ez[idx];
-                    v = decay * before + gain * curl;
-                    if ((long long)idx == a.src) {
-                        // soft current: ε dE/dt = ∇×H − J, with the σ term's semi-implicit divisor
-                        const double e = a.eps_src, ss = a.sig_src;
-                        v = (Real)((double)v - (dt / e) / (1.0 + (ss * dt / (2.0 * e))) * jsrc);
-                        acc[1] += -(dt * a.volume) * jsrc * (0.5 * ((double)before + (double)v));
-                    }
-                    const double mid = 0.5 * ((double)before + (double)v);
-                    acc[0] += s * mid * mid * dt * a.volume;
-                }
-                if (a.solid && touches_solid(a.solid, nx, ny, nz, i - 1, i, j - 1, j, k, k)) v = Real(0);
-                a.ez[idx] = v;
-            }
-            hy_km = hy_k;
-            hx_km = hx_k;
-        }
-    }
-    if (finish_blocks<2>(acc, a.partials, a.nblocks, &st->counter) && linear_tid() == 0) {
-        st->dissipated += fmax(acc[0], 0.0);
-        // The invariant of this step was taken before this step's electric update, so the work
-        // that update did is booked against the next step's invariant.
-        st->work_booked = st->work;
-        st->work += acc[1];
-        double total = 0.0, scale = 0.0;
-        ledger_add(total, scale, st->invariant);
-        ledger_add(total, scale, st->dissipated);
-        if (a.with_source) ledger_add(total, scale, -st->work_booked);
-        st->part[0] = st->invariant;
-        st->part[1] = st->dissipated;
-        st->part[2] = -st->work_booked;
-        audit_and_commit(st, total, scale);
-    }
+// The edges of lattice node (i, j, k) that touch a solid cell (cavity.rs:304-331): bits 1, 2, 4 for ex, ey,
+// ez, one byte a node, i + (nx + 1)·(j + (ny + 1)·k), formed on the host when the obstacles change. Four
+// cells' flags an edge, twelve byte loads and their bounds a node, had taken nearly half of an obstructed
+// cavity's step: 68 × 77 × 94 cells in f64 ran 42.7 µs a step with them and 24.1 with this.
+__device__ __forceinline__ unsigned solid_edges(const uint8_t* edges, int nx, int ny, int i, int j, int k) {
+    return edges[(size_t)i + (size_t)(nx + 1) * ((size_t)j + (size_t)(ny + 1) * (size_t)k)];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -361,7 +219,7 @@ struct YeeStepArgs {
     const double* __restrict__ sig0;
     const double* __restrict__ sig1;
     const double* __restrict__ sig2;
-    const uint8_t* __restrict__ solid;
+    const uint8_t* __restrict__ solid;  // edges by lattice node (solid_edges); null without obstacles
     int src_i, src_j, src_k;  // the Ez edge with a soft current (extension); src_i < 0: none
     const double* __restrict__ current;
     long long ncurrent;
@@ -655,6 +513,9 @@ static __global__ void __launch_bounds__(256, YeeDepth<Real>::min_blocks) yee_st
                 if (fz) { muz = a.mu2[own_h[5]]; cz = a.cch[2][own_h[5]]; }
             }
         }
+        unsigned solid = 0;
+        if constexpr (SOLID)
+            if (compute && in_x && in_y) solid = solid_edges(a.solid, nx, ny, i, j, k);
         const Real hxn = wx - cx * ((S0.ez[ty + 2][tx + 1] - ez0) - (S1.ey[ty + 1][tx + 1] - ey0));
         const Real hyn = wy - cy * ((S1.ex[ty + 1][tx + 1] - ex0) - (S0.ez[ty + 1][tx + 2] - ez0));
         const Real hzn = wz - cz * ((S0.ey[ty + 1][tx + 2] - ey0) - (S0.ex[ty + 2][tx + 1] - ex0));
@@ -749,9 +610,9 @@ static __global__ void __launch_bounds__(256, YeeDepth<Real>::min_blocks) yee_st
                 acc[2] += (lz && in_x && in_y && zin) ? s2 * mz * mz * dt * a.volume : 0.0;
             }
             if constexpr (SOLID) {
-                if (touches_solid(a.solid, nx, ny, nz, i, i, j - 1, j, k - 1, k)) vx = Real(0);
-                if (touches_solid(a.solid, nx, ny, nz, i - 1, i, j, j, k - 1, k)) vy = Real(0);
-                if (touches_solid(a.solid, nx, ny, nz, i - 1, i, j - 1, j, k, k)) vz = Real(0);
+                if (solid & 1) vx = Real(0);
+                if (solid & 2) vy = Real(0);
+                if (solid & 4) vz = Real(0);
             }
             if (i < nx && in_y) a.neu[0][own_h[0]] = vx;
             if (in_x && j < ny) a.neu[1][own_h[1]] = vy;

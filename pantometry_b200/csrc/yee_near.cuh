@@ -166,9 +166,7 @@ __device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4], DevS
             acc[2] += a.sig0 * m * m * a.dt * a.volume;
         }
         if constexpr (SOLID) {
-            const bool hit = q == 0   ? touches_solid(a.solid, nx, ny, nz, i, i, j - 1, j, k - 1, k)
-                             : q == 1 ? touches_solid(a.solid, nx, ny, nz, i - 1, i, j, j, k - 1, k)
-                                      : touches_solid(a.solid, nx, ny, nz, i - 1, i, j - 1, j, k, k);
+            const bool hit = (solid_edges(a.solid, nx, ny, i, j, k) >> q) & 1;
             if (hit) v = 0.0;
         }
         a.nneu[near_box(a, q, i, j, k)] = v;
@@ -209,9 +207,7 @@ __device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4], DevS
             acc[2] += a.sig0 * mnew * mnew * a.dt * a.volume - a.sig0 * mold * mold * a.dt * a.volume;
         }
         if constexpr (SOLID) {
-            const bool hit = q == 0   ? touches_solid(a.solid, nx, ny, nz, i, i, j - 1, j, k - 1, k)
-                             : q == 1 ? touches_solid(a.solid, nx, ny, nz, i - 1, i, j, j, k - 1, k)
-                                      : touches_solid(a.solid, nx, ny, nz, i - 1, i, j - 1, j, k, k);
+            const bool hit = (solid_edges(a.solid, nx, ny, i, j, k) >> q) & 1;
             if (hit) v = 0.0f;
         }
         out[n] = v;

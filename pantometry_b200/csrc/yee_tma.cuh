@@ -327,6 +327,9 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
                 gy = (in_x && by) ? GY[h][ty][tx] : gain0;
                 gz = (in_x && in_y && zin) ? GZ[h][ty][tx] : gain0;
             }
+            unsigned solid = 0;
+            if constexpr (SOLID)
+                if (compute && in_x && in_y) solid = solid_edges(a.solid, nx, ny, i, j, k);
             YeeHp<float>* hq = hp + hpar;
             // ---- 1. H⁺ (cavity.rs:1346-1379) on own faces
             const bool fx = in_x && by && zin, fy = bx && in_y && zin, fz = bx && by;
@@ -404,9 +407,9 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
                     acc[2] += (lz && in_x && in_y && zin) ? sig0 * mz * mz * dt * a.volume : 0.0;
                 }
                 if constexpr (SOLID) {
-                    if (touches_solid(a.solid, nx, ny, nz, i, i, j - 1, j, k - 1, k)) vx = 0.0f;
-                    if (touches_solid(a.solid, nx, ny, nz, i - 1, i, j, j, k - 1, k)) vy = 0.0f;
-                    if (touches_solid(a.solid, nx, ny, nz, i - 1, i, j - 1, j, k, k)) vz = 0.0f;
+                    if (solid & 1) vx = 0.0f;
+                    if (solid & 2) vy = 0.0f;
+                    if (solid & 4) vz = 0.0f;
                 }
                 if (bx && in_y) a.neu[0][n] = vx;
                 if (in_x && by) a.neu[1][n] = vy;
