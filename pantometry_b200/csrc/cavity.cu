@@ -362,10 +362,16 @@ struct Cavity : Handle {
     pm_status upload_edges() {
         const size_t sy = (size_t)nx + 1, sz = sy * ((size_t)ny + 1);
         std::vector<uint8_t> e(sz * ((size_t)nz + 1), 0);
+        for (int a = 0; a < 3; ++a) { solid_lo[a] = std::max(nx, std::max(ny, nz)); solid_hi[a] = -1; }
         for (int k = 0; k < nz; ++k)
             for (int j = 0; j < ny; ++j)
                 for (int i = 0; i < nx; ++i) {
                     if (!solid[i + (size_t)nx * (j + (size_t)ny * k)]) continue;
+                    const int at[3] = {i, j, k};
+                    for (int a = 0; a < 3; ++a) {
+                        solid_lo[a] = std::min(solid_lo[a], at[a]);
+                        solid_hi[a] = std::max(solid_hi[a], at[a]);
+                    }
                     uint8_t* n = &e[i + sy * j + sz * k];
                     for (size_t q : {size_t(0), sy, sz, sy + sz}) n[q] |= 1;
                     for (size_t q : {size_t(0), size_t(1), sz, 1 + sz}) n[q] |= 2;
@@ -385,7 +391,16 @@ struct Cavity : Handle {
     // history, and only then zeroes the obstacles' edges (cavity.rs:1497-1499, 1159-1163). The
     // step kernels then leave those edges alone, the walls run, E is copied to `stale` (the history
     // lives there from then on) and yee_enforce_solid zeroes the edges.
-    bool solid_after_walls() const { return any_solid && open_or_magnetic(); }
+    // Obstacles whose edges stay off such a wall and off the plane inside it are out of the walls'
+    // reach and out of their history, so the step kernels zero them as they do in a conducting box.
+    int solid_lo[3] = {0, 0, 0}, solid_hi[3] = {0, 0, 0};  // the solid cells' least and greatest indices
+    bool solid_after_walls() const {
+        if (!any_solid) return false;
+        const int n[3] = {nx, ny, nz};
+        for (int a = 0; a < 3; ++a)
+            if ((boundary[2 * a] != 0 && solid_lo[a] <= 1) || (boundary[2 * a + 1] != 0 && solid_hi[a] >= n[a] - 2)) return true;
+        return false;
+    }
     pm_status ensure_stale() {
         for (int q = 0; q < 3; ++q) {
             const size_t bytes = dcount(q) * esize();
@@ -405,7 +420,7 @@ struct Cavity : Handle {
         return PM_OK;
     }
     // The walls after the step from `par` into `par ^ 1` (cavity.rs:1074-1164): magnetic mirrors,
-    // then open walls by Mur (or held at zero before any history exists), one wall at a time.
+    // then open walls by Mur (or held at zero before any history exists).
     template <typename Real>
     YeeWallArgs<Real> wall_args(int par, bool stale_history) const {
         YeeWallArgs<Real> a{};
@@ -435,20 +450,27 @@ struct Cavity : Handle {
         YeeWallArgs<Real> a = wall_args<Real>(par, stale_history);
         const double c_dt = wave_speed() * dt;
         a.k = (Real)((c_dt - dx) / (c_dt + dx));  // cavity.rs:1075-1078
-        for (int w = 0; w < 6; ++w) {
-            if (boundary[w] != 1) continue;
-            a.wall = w;
-            a.kind = 1;
-            cudaError_t e = launch_yee_walls<Real>(a, s);
-            if (e != cudaSuccess) return e;
-        }
-        for (int w = 0; w < 6; ++w) {
-            if (boundary[w] != 2) continue;
-            a.wall = w;
-            a.kind = prev ? 2 : 3;
-            cudaError_t e = launch_yee_walls<Real>(a, s);
-            if (e != cudaSuccess) return e;
-        }
+        const int n[3] = {nx, ny, nz};
+        auto launch = [&](auto&& ours) {  // the walls `ours` names, in one launch
+            a.first[0] = 0;
+            for (int w = 0; w < 6; ++w) {
+                a.kind[w] = !ours(w) ? 0 : boundary[w] == 1 ? 1 : prev ? 2 : 3;
+                const unsigned u = (unsigned)n[w < 2 ? 1 : 0], v = (unsigned)n[w < 4 ? 2 : 1];
+                a.first[w + 1] = a.first[w] + (a.kind[w] ? u * (v + 1) + (u + 1) * v : 0);
+            }
+            return launch_yee_walls<Real>(a, s);
+        };
+        // an axis of one cell: its walls' inner neighbours lie on the opposite wall, so one wall at a
+        // time, in the reference's order (magnetic walls, then open ones)
+        bool thin = false;
+        for (int w = 0; w < 6; ++w) thin = thin || (boundary[w] != 0 && n[w >> 1] < 2);
+        if (!thin) return launch([&](int w) { return boundary[w] != 0; });
+        for (int kind : {1, 2})
+            for (int w = 0; w < 6; ++w) {
+                if (boundary[w] != kind) continue;
+                cudaError_t e = launch([&](int one) { return one == w; });
+                if (e != cudaSuccess) return e;
+            }
         return cudaSuccess;
     }
     // One step from `par`, its walls included.

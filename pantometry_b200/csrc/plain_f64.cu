@@ -95,7 +95,7 @@ cudaError_t launch_yee_enforce_solid<double>(const YeeWallArgs<double>& a, const
 }
 template <>
 cudaError_t launch_yee_walls<double>(const YeeWallArgs<double>& a, cudaStream_t s) {
-    yee_walls<double><<<kMeasureBlocks, 256, 0, s>>>(a);
+    yee_walls<double><<<std::min((a.first[6] + 255u) / 256u, (unsigned)kMeasureBlocks), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 template <>
