@@ -73,7 +73,6 @@ struct Cavity : Handle {
     // kNearWidth³ lattice nodes around the source edge, one set per parity. Kept when the cavity
     // is TMA-staged FP32 with a source and the box, with the ring of edges on its high sides,
     // lies one node or more inside the walls (near_w = kNearWidth); otherwise near_w = 0.
-    static constexpr int kNearWidth = 5;
     int near_x0 = 0, near_y0 = 0, near_z0 = 0, near_w = 0;
     DBuf dnear[2];
     bool near_dirty = true;  // the stored field changed outside a step: seed the box from it
@@ -485,8 +484,9 @@ struct Cavity : Handle {
             YeeStepArgs<float> t = targs(par, h);
             if (after) t.solid = nullptr;
             if (near_on()) {
-                // the box's terms and the source are the step's last block's; it closes the books
+                // the box's terms and the source are those of the grid's block 0, which takes no tiles
                 const YeeNearArgs n = nargs(par, h, t);
+                t.nblocks = std::max(1u, std::min(t.nblocks, wave_of(yee_tma_kernel_id(!uniform, yshape)) - 1));
                 t.nb_x0 = near_x0; t.nb_y0 = near_y0; t.nb_z0 = near_z0; t.nb_w = near_w;
                 t.src_i = t.src_j = t.src_k = -1;
                 e = launch_yee_tma(t, L, maps[par], yshape, s, n);
@@ -576,7 +576,7 @@ struct Cavity : Handle {
         n.src_i = t.src_i; n.src_j = t.src_j; n.src_k = t.src_k;
         n.current = t.current; n.ncurrent = t.ncurrent;
         n.eps_src = t.eps_src; n.sig_src = t.sig_src;
-        n.dt = h; n.volume = t.volume; n.g = t.g; n.eps_u = t.eps_u; n.mu_u = t.mu_u;
+        n.dt = h; n.volume = t.volume;
         return n;
     }
     // The box's f64 values from the stored field of the present parity.

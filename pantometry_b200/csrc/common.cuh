@@ -37,6 +37,12 @@ __host__ __device__ inline Tiles make_tiles(int nx, int ny, int nz, int zc, int 
     return t;
 }
 
+// A compile-time flag as an argument.
+template <bool B>
+struct Flag {
+    static constexpr bool value = B;
+};
+
 // Asynchronous global → shared copies (cp.async, sm_80 and later): each thread queues element
 // copies for planes ahead of the one it computes, so the bytes in flight are set by the ring of
 // shared-memory stages rather than by registers or thread count.

@@ -62,11 +62,6 @@ struct alignas(16) EnsBrickInfo {
 };
 static_assert(sizeof(EnsBrickInfo) == 128, "one record is one 128-byte bulk copy");
 
-template <bool B>
-struct Flag {
-    static constexpr bool value = B;
-};
-
 constexpr unsigned kEnsHoldBlocks = 16384;  // blocks whose stop flags fit the shared bitmask
 
 struct EnsTmaArgs {

@@ -143,7 +143,7 @@ static cudaError_t launch_yee_tma_shape(const YeeStepArgs<float>& a, unsigned L,
     const int smem = (int)yee_tma_smem_bytes_for<P, MEDIA>(S);
     auto k = a.solid ? (a.wall_split ? yee_tma_step<P, S, true, MEDIA, MINB, true> : yee_tma_step<P, S, true, MEDIA, MINB, false>)
                      : (a.wall_split ? yee_tma_step<P, S, false, MEDIA, MINB, true> : yee_tma_step<P, S, false, MEDIA, MINB, false>);
-    return launch_smem(k, a.nblocks, tile_block(), smem, s, a, L, m, n);
+    return launch_smem(k, a.nblocks + (a.nb_w > 0 ? 1u : 0u), tile_block(), smem, s, a, L, m, n);
 }
 cudaError_t launch_yee_tma(const YeeStepArgs<float>& a, unsigned L, const YeeMaps& m, int shape, cudaStream_t s,
                            const YeeNearArgs& n) {

@@ -237,8 +237,8 @@ struct YeeStepArgs {
     const Real* __restrict__ cch[3];
     int lossless, mu_var;
     // FP32 TMA form only: a box of nb_w³ lattice nodes from (nb_x0, nb_y0, nb_z0) whose six
-    // components the kernel's last block steps again in f64 (yee_near_body) once the grid's cells
-    // are in; the box's energy terms are left to it, and it closes the books. nb_w = 0: none.
+    // components block 0 steps in f64 (yee_near_block) beside the tiles; the tiles leave it the box's
+    // edges, faces and energy terms and the ring's edges. nb_w = 0: none.
     int nb_x0, nb_y0, nb_z0, nb_w;
     // FP32 TMA form only: the tiles cover [0, nx) × [0, ny) of the lattice and the last column and
     // row are stepped by the wall pass (yee_tma_wall_pass). 0: the tiles cover the whole lattice.

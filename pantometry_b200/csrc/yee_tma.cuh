@@ -93,9 +93,9 @@ __device__ __forceinline__ void yee_tma_at(YeeTmaCursor& c, const Tiles& T, unsi
     c.k1 = min(T.nz, c.k0 + T.zc);  // T.nz = nz + 1 lattice planes
     c.kb = c.k0 > 0 ? c.k0 - 1 : 0;
 }
-__device__ __forceinline__ void yee_tma_next(YeeTmaCursor& c, const Tiles& T, int planes) {
+__device__ __forceinline__ void yee_tma_next(YeeTmaCursor& c, const Tiles& T, int planes, unsigned stride) {
     c.kb += planes;
-    if (c.kb >= c.k1) yee_tma_at(c, T, c.t + gridDim.x);
+    if (c.kb >= c.k1) yee_tma_at(c, T, c.t + stride);
 }
 
 template <int P, bool MEDIA>
@@ -138,8 +138,9 @@ __device__ __forceinline__ void yee_tma_close(DevState* st, const double (&acc)[
     audit_and_commit(st, total, scale);
 }
 
-// The near field of a soft current, kept in f64 (yee_near.cuh): its arguments, and the last
-// block's work on it after the grid's sums are in.
+// The near field of a soft current, kept in f64 (yee_near.cuh): its arguments, and the work of the
+// grid's block 0 on it.
+constexpr int kNearWidth = 5;  // lattice nodes of the box along each axis
 struct YeeNearArgs {
     const float* old[6];    // ex ey ez hx hy hz at step n, padded lattice
     float* neu[6];          // at n + 1, already stepped by yee_tma_step
@@ -157,10 +158,20 @@ struct YeeNearArgs {
     int src_i, src_j, src_k;
     const double* current;
     long long ncurrent;
-    double eps_src, sig_src, dt, volume, g, eps_u, mu_u;
+    double eps_src, sig_src, dt, volume;
 };
+struct YeeNearShared;
 template <bool SOLID>
-__device__ void yee_near_body(const YeeNearArgs& a, const double (&tma)[4], DevState* st);
+__device__ void yee_near_block(YeeNearShared& sh, long long step, double (&acc)[4]);
+// The near-field nodes a tile leaves to block 0: bits 1, 2, 4 where the node's ex, ey, ez is one the box or
+// its ring forms again (yee_near.cuh), 8 where the node is in the box (its faces and energies too).
+__device__ __forceinline__ unsigned near_left(int di, int dj, int dk, int w) {  // the node from the box's first
+    const unsigned n = (unsigned)w;
+    const bool i = (unsigned)di < n, j = (unsigned)dj < n, k = (unsigned)dk < n;
+    const bool im = (unsigned)(di - 1) < n, jm = (unsigned)(dj - 1) < n, km = (unsigned)(dk - 1) < n;
+    return (i && ((j && (k || km)) || (jm && k)) ? 1u : 0u) | (j && ((i && (k || km)) || (im && k)) ? 2u : 0u) |
+           (k && ((i && (j || jm)) || (im && j)) ? 4u : 0u) | (i && j && k ? 8u : 0u);
+}
 
 // One face of H⁺ (cavity.rs:1346-1379): was − (g/μ)·((a₁ − a₀) − (b₁ − b₀)). The tiles and the
 // wall pass below form every face through this one expression, so the two agree bit for bit.
@@ -256,13 +267,16 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
     __syncthreads();
 
     YeeTmaCursor pf, cc;
-    yee_tma_at(cc, T, blockIdx.x);
+    // with a near-field box block 0 steps the box, beside the tiles, and takes none of them
+    const bool near_block = a.nb_w > 0 && blockIdx.x == 0;
+    const unsigned tiles0 = blockIdx.x - (a.nb_w > 0 ? 1u : 0u), stride = gridDim.x - (a.nb_w > 0 ? 1u : 0u);
+    yee_tma_at(cc, T, near_block ? 0xffffffffu : tiles0);
     int issued = 0;
     if (tid == 0) {
-        yee_tma_at(pf, T, blockIdx.x);
+        pf = cc;
         for (; issued < S - 1 && pf.valid; ++issued) {
             yee_tma_issue<P, MEDIA>(m, ring_base + issued * Lay::BYTES, bar_base + 8 * issued, pf);
-            yee_tma_next(pf, T, P);
+            yee_tma_next(pf, T, P, stride);
         }
     }
     const float ch = a.ch;
@@ -284,7 +298,7 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
             const int fill = (it + S - 1) % S;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             yee_tma_issue<P, MEDIA>(m, ring_base + fill * Lay::BYTES, bar_base + 8 * fill, pf);
-            yee_tma_next(pf, T, P);
+            yee_tma_next(pf, T, P, stride);
             ++issued;
         }
         const unsigned char* sb = yee_tma_smem + slot * Lay::BYTES;
@@ -303,126 +317,140 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
         const bool in_x = SPLIT || i <= nx, in_y = SPLIT || j <= ny, bx = SPLIT || i < nx, by = SPLIT || j < ny;
         // node-centred half weights of the boundary samples (cavity.rs:766-772)
         const float hi = (i == 0 || (!SPLIT && i == nx)) ? 0.5f : 1.0f, hj = (j == 0 || (!SPLIT && j == ny)) ? 0.5f : 1.0f;
-        // the column crosses the f64 near-field box (nb_w = 0: no box, never)
-        const bool box_xy = (unsigned)(i - a.nb_x0) < (unsigned)a.nb_w && (unsigned)(j - a.nb_y0) < (unsigned)a.nb_w;
         // this stage's energy products of the thread's cells per component, the z weight in each:
         // Σ hk ex², Σ hk ey², Σ ez² (with MEDIA each over its gain), Σ hx⁺hx⁻, Σ hy⁺hy⁻, Σ hk hz⁺hz⁻;
         // the x and y weights are applied once a stage
         float sx = 0.0f, sy = 0.0f, sz = 0.0f, mx = 0.0f, my = 0.0f, mz = 0.0f;
+        auto planes = [&](auto near_tag) {
 #pragma unroll
-        for (int h = 0; h < P; ++h) {
-            const int k = cc.kb + h;
-            if (k >= cc.k1) break;
-            const bool compute = k >= cc.k0;  // else the plane below the chunk: H⁺ only
-            const bool zin = k < nz;
-            const float hk = (k == 0 || k == nz) ? 0.5f : 1.0f;
-            // a node of the near-field box: its energy terms are the box kernel's, in f64
-            const bool inbox = box_xy && (unsigned)(k - a.nb_z0) < (unsigned)a.nb_w;
-            const unsigned n = (unsigned)i + L * ((unsigned)j + ny1 * (unsigned)k);
-            // the gains of the thread's own edges; at a position the component does not have (the
-            // padding, or the fill outside the lattice) the uniform gain, never read as a value
-            float gx = gain0, gy = gain0, gz = gain0;
-            if constexpr (MEDIA) {
-                gx = (bx && in_y) ? GX[h][ty][tx] : gain0;
-                gy = (in_x && by) ? GY[h][ty][tx] : gain0;
-                gz = (in_x && in_y && zin) ? GZ[h][ty][tx] : gain0;
-            }
-            unsigned solid = 0;
-            if constexpr (SOLID)
-                if (compute && in_x && in_y) solid = solid_edges(a.solid, nx, ny, i, j, k);
-            YeeHp<float>* hq = hp + hpar;
-            // ---- 1. H⁺ (cavity.rs:1346-1379) on own faces
-            const bool fx = in_x && by && zin, fy = bx && in_y && zin, fz = bx && by;
-            const float wx = HX[h][ty + 1][tx], wy = HY[h][ty][tx + 4], wz = HZ[h][ty + 1][tx + 4];
-            const float ex0 = EX[h][ty + 1][tx + 4], ey0 = EY[h][ty + 1][tx + 4], ez0 = EZ[h][ty + 1][tx + 4];
-            const float hxn = yee_face_f32(wx, ch, EZ[h][ty + 2][tx + 4], ez0, EY[h + 1][ty + 1][tx + 4], ey0);
-            const float hyn = yee_face_f32(wy, ch, EX[h + 1][ty + 1][tx + 4], ex0, EZ[h][ty + 1][tx + 5], ez0);
-            const float hzn = yee_face_f32(wz, ch, EY[h][ty + 1][tx + 5], ey0, EX[h][ty + 2][tx + 4], ex0);
-            hq->hx[ty + 1][tx] = hxn;
-            hq->hy[ty][tx + 1] = hyn;
-            hq->hz[ty + 1][tx + 1] = hzn;
-            if (compute) {
-                if (fx) a.neu[3][n] = hxn;
-                if (fy) a.neu[4][n] = hyn;
-                if (fz) a.neu[5][n] = hzn;
-                // ½μ H⁻·H⁺ (cavity.rs:854-905) and ½εEⁿ² (cavity.rs:776-847), weights only. No
-                // mask is needed: at a lattice position a component does not have, its old value
-                // (padding, or the fill outside the lattice) is exactly zero, so its E term and
-                // its H⁻·H⁺ term are zero.
-                if (!inbox) {
-                    mx = fmaf(hxn, wx, mx);
-                    my = fmaf(hyn, wy, my);
-                    mz = fmaf(hk * hzn, wz, mz);
-                    if constexpr (MEDIA) {  // 1/g to within 2 ulp: the terms are f32 roundings already
-                        sx += __fdividef((hk * ex0) * ex0, gx);
-                        sy += __fdividef((hk * ey0) * ey0, gy);
-                        sz += __fdividef(ez0 * ez0, gz);
-                    } else {
-                        sx = fmaf(hk * ex0, ex0, sx);
-                        sy = fmaf(hk * ey0, ey0, sy);
-                        sz = fmaf(ez0, ez0, sz);
+            for (int h = 0; h < P; ++h) {
+                const int k = cc.kb + h;
+                if (k >= cc.k1) break;
+                const bool compute = k >= cc.k0;  // else the plane below the chunk: H⁺ only
+                const bool zin = k < nz;
+                const float hk = (k == 0 || k == nz) ? 0.5f : 1.0f;
+                unsigned left = 0;  // what block 0 forms of this node
+                if constexpr (decltype(near_tag)::value) left = near_left(i - a.nb_x0, j - a.nb_y0, k - a.nb_z0, a.nb_w);
+                const bool inbox = left & 8;  // its faces and energy terms are the box's, in f64
+                const unsigned n = (unsigned)i + L * ((unsigned)j + ny1 * (unsigned)k);
+                // the gains of the thread's own edges; at a position the component does not have (the
+                // padding, or the fill outside the lattice) the uniform gain, never read as a value
+                float gx = gain0, gy = gain0, gz = gain0;
+                if constexpr (MEDIA) {
+                    gx = (bx && in_y) ? GX[h][ty][tx] : gain0;
+                    gy = (in_x && by) ? GY[h][ty][tx] : gain0;
+                    gz = (in_x && in_y && zin) ? GZ[h][ty][tx] : gain0;
+                }
+                unsigned solid = 0;
+                if constexpr (SOLID)
+                    if (compute && in_x && in_y) solid = solid_edges(a.solid, nx, ny, i, j, k);
+                YeeHp<float>* hq = hp + hpar;
+                // ---- 1. H⁺ (cavity.rs:1346-1379) on own faces
+                const bool fx = in_x && by && zin, fy = bx && in_y && zin, fz = bx && by;
+                const float wx = HX[h][ty + 1][tx], wy = HY[h][ty][tx + 4], wz = HZ[h][ty + 1][tx + 4];
+                const float ex0 = EX[h][ty + 1][tx + 4], ey0 = EY[h][ty + 1][tx + 4], ez0 = EZ[h][ty + 1][tx + 4];
+                const float hxn = yee_face_f32(wx, ch, EZ[h][ty + 2][tx + 4], ez0, EY[h + 1][ty + 1][tx + 4], ey0);
+                const float hyn = yee_face_f32(wy, ch, EX[h + 1][ty + 1][tx + 4], ex0, EZ[h][ty + 1][tx + 5], ez0);
+                const float hzn = yee_face_f32(wz, ch, EY[h][ty + 1][tx + 5], ey0, EX[h][ty + 2][tx + 4], ex0);
+                hq->hx[ty + 1][tx] = hxn;
+                hq->hy[ty][tx + 1] = hyn;
+                hq->hz[ty + 1][tx + 1] = hzn;
+                if (compute) {
+                    if (fx && !inbox) a.neu[3][n] = hxn;
+                    if (fy && !inbox) a.neu[4][n] = hyn;
+                    if (fz && !inbox) a.neu[5][n] = hzn;
+                    // ½μ H⁻·H⁺ (cavity.rs:854-905) and ½εEⁿ² (cavity.rs:776-847), weights only. No
+                    // mask is needed: at a lattice position a component does not have, its old value
+                    // (padding, or the fill outside the lattice) is exactly zero, so its E term and
+                    // its H⁻·H⁺ term are zero.
+                    if (!inbox) {
+                        mx = fmaf(hxn, wx, mx);
+                        my = fmaf(hyn, wy, my);
+                        mz = fmaf(hk * hzn, wz, mz);
+                        if constexpr (MEDIA) {  // 1/g to within 2 ulp: the terms are f32 roundings already
+                            sx += __fdividef((hk * ex0) * ex0, gx);
+                            sy += __fdividef((hk * ey0) * ey0, gy);
+                            sz += __fdividef(ez0 * ez0, gz);
+                        } else {
+                            sx = fmaf(hk * ex0, ex0, sx);
+                            sy = fmaf(hk * ey0, ey0, sy);
+                            sz = fmaf(ez0, ez0, sz);
+                        }
+                    }
+                    // halo faces, one line per warp so the barrier waits on no warp doing twice the
+                    // work: the y0 − 1 row of hx (warp 7) and of hz (warp 6), the x0 − 1 column of hz
+                    // (warp 5, rows y0 − 1 .. y0 + 7) and of hy (warp 4, rows y0 .. y0 + 7)
+                    if (ty == 7) {
+                        hq->hx[0][tx] = yee_face_f32(HX[h][0][tx], ch, EZ[h][1][tx + 4], EZ[h][0][tx + 4], EY[h + 1][0][tx + 4], EY[h][0][tx + 4]);
+                    } else if (ty == 6) {
+                        hq->hz[0][tx + 1] = yee_face_f32(HZ[h][0][tx + 4], ch, EY[h][0][tx + 5], EY[h][0][tx + 4], EX[h][1][tx + 4], EX[h][0][tx + 4]);
+                    } else if (ty == 5 && tx < 9) {
+                        const int r = tx;
+                        hq->hz[r][0] = yee_face_f32(HZ[h][r][3], ch, EY[h][r][4], EY[h][r][3], EX[h][r + 1][3], EX[h][r][3]);
+                    } else if (ty == 4 && tx >= 1 && tx < 9) {
+                        const int r = tx;
+                        hq->hy[r - 1][0] = yee_face_f32(HY[h][r - 1][3], ch, EX[h + 1][r][3], EX[h][r][3], EZ[h][r][4], EZ[h][r][3]);
                     }
                 }
-                // halo faces, one line per warp so the barrier waits on no warp doing twice the
-                // work: the y0 − 1 row of hx (warp 7) and of hz (warp 6), the x0 − 1 column of hz
-                // (warp 5, rows y0 − 1 .. y0 + 7) and of hy (warp 4, rows y0 .. y0 + 7)
-                if (ty == 7) {
-                    hq->hx[0][tx] = yee_face_f32(HX[h][0][tx], ch, EZ[h][1][tx + 4], EZ[h][0][tx + 4], EY[h + 1][0][tx + 4], EY[h][0][tx + 4]);
-                } else if (ty == 6) {
-                    hq->hz[0][tx + 1] = yee_face_f32(HZ[h][0][tx + 4], ch, EY[h][0][tx + 5], EY[h][0][tx + 4], EX[h][1][tx + 4], EX[h][0][tx + 4]);
-                } else if (ty == 5 && tx < 9) {
-                    const int r = tx;
-                    hq->hz[r][0] = yee_face_f32(HZ[h][r][3], ch, EY[h][r][4], EY[h][r][3], EX[h][r + 1][3], EX[h][r][3]);
-                } else if (ty == 4 && tx >= 1 && tx < 9) {
-                    const int r = tx;
-                    hq->hy[r - 1][0] = yee_face_f32(HY[h][r - 1][3], ch, EX[h + 1][r][3], EX[h][r][3], EZ[h][r][4], EZ[h][r][3]);
+                __syncthreads();
+                // ---- 2. Eⁿ⁺¹ on own edges (cavity.rs:1383-1452): interior by the semi-implicit update,
+                // conducting walls 0 (cavity.rs:1239-1293), edges touching a solid cell 0 (cavity.rs:304-331)
+                if (compute) {
+                    const bool ix = i >= 1 && bx, iy = j >= 1 && by, iz = k >= 1 && k < nz;
+                    const float cex = (hzn - hq->hz[ty][tx + 1]) - (hyn - hy_below);  // own H⁺ from registers
+                    const float cey = (hxn - hx_below) - (hzn - hq->hz[ty + 1][tx]);
+                    const float cez = (hyn - hq->hy[ty][tx]) - (hxn - hq->hx[ty][tx]);
+                    float vx = dec0 * ex0 + gx * cex;
+                    float vy = dec0 * ey0 + gy * cey;
+                    float vz = dec0 * ez0 + gz * cez;
+                    if (i == a.src_i && j == a.src_j && k == a.src_k) {
+                        // soft current: ε dE/dt = ∇×H − J, with the σ term's semi-implicit divisor
+                        const double e = a.eps_src, ss = a.sig_src;
+                        vz = (float)((double)vz - (dt / e) / (1.0 + (ss * dt / (2.0 * e))) * jsrc);
+                        acc[3] += -(dt * a.volume) * jsrc * (0.5 * ((double)ez0 + (double)vz));
+                    }
+                    const bool lx = iy && iz, ly = ix && iz, lz = ix && iy;  // interior edges
+                    vx = lx ? vx : 0.0f;
+                    vy = ly ? vy : 0.0f;
+                    vz = lz ? vz : 0.0f;
+                    if (lossy) {
+                        const double mx = 0.5 * ((double)ex0 + (double)vx), my = 0.5 * ((double)ey0 + (double)vy),
+                                     mz = 0.5 * ((double)ez0 + (double)vz);
+                        acc[2] += (lx && bx && in_y && !(left & 1)) ? sig0 * mx * mx * dt * a.volume : 0.0;
+                        acc[2] += (ly && in_x && by && !(left & 2)) ? sig0 * my * my * dt * a.volume : 0.0;
+                        acc[2] += (lz && in_x && in_y && zin && !(left & 4)) ? sig0 * mz * mz * dt * a.volume : 0.0;
+                    }
+                    if constexpr (SOLID) {
+                        if (solid & 1) vx = 0.0f;
+                        if (solid & 2) vy = 0.0f;
+                        if (solid & 4) vz = 0.0f;
+                    }
+                    if (bx && in_y && !(left & 1)) a.neu[0][n] = vx;
+                    if (in_x && by && !(left & 2)) a.neu[1][n] = vy;
+                    if (in_x && in_y && zin && !(left & 4)) a.neu[2][n] = vz;
                 }
+                hx_below = hxn;
+                hy_below = hyn;
+                hpar ^= 1;
             }
-            __syncthreads();
-            // ---- 2. Eⁿ⁺¹ on own edges (cavity.rs:1383-1452): interior by the semi-implicit update,
-            // conducting walls 0 (cavity.rs:1239-1293), edges touching a solid cell 0 (cavity.rs:304-331)
-            if (compute) {
-                const bool ix = i >= 1 && bx, iy = j >= 1 && by, iz = k >= 1 && k < nz;
-                const float cex = (hzn - hq->hz[ty][tx + 1]) - (hyn - hy_below);  // own H⁺ from registers
-                const float cey = (hxn - hx_below) - (hzn - hq->hz[ty + 1][tx]);
-                const float cez = (hyn - hq->hy[ty][tx]) - (hxn - hq->hx[ty][tx]);
-                float vx = dec0 * ex0 + gx * cex;
-                float vy = dec0 * ey0 + gy * cey;
-                float vz = dec0 * ez0 + gz * cez;
-                if (i == a.src_i && j == a.src_j && k == a.src_k) {
-                    // soft current: ε dE/dt = ∇×H − J, with the σ term's semi-implicit divisor
-                    const double e = a.eps_src, ss = a.sig_src;
-                    vz = (float)((double)vz - (dt / e) / (1.0 + (ss * dt / (2.0 * e))) * jsrc);
-                    acc[3] += -(dt * a.volume) * jsrc * (0.5 * ((double)ez0 + (double)vz));
-                }
-                const bool lx = iy && iz, ly = ix && iz, lz = ix && iy;  // interior edges
-                vx = lx ? vx : 0.0f;
-                vy = ly ? vy : 0.0f;
-                vz = lz ? vz : 0.0f;
-                if (lossy && !inbox) {
-                    const double mx = 0.5 * ((double)ex0 + (double)vx), my = 0.5 * ((double)ey0 + (double)vy),
-                                 mz = 0.5 * ((double)ez0 + (double)vz);
-                    acc[2] += (lx && bx && in_y) ? sig0 * mx * mx * dt * a.volume : 0.0;
-                    acc[2] += (ly && in_x && by) ? sig0 * my * my * dt * a.volume : 0.0;
-                    acc[2] += (lz && in_x && in_y && zin) ? sig0 * mz * mz * dt * a.volume : 0.0;
-                }
-                if constexpr (SOLID) {
-                    if (solid & 1) vx = 0.0f;
-                    if (solid & 2) vy = 0.0f;
-                    if (solid & 4) vz = 0.0f;
-                }
-                if (bx && in_y) a.neu[0][n] = vx;
-                if (in_x && by) a.neu[1][n] = vy;
-                if (in_x && in_y && zin) a.neu[2][n] = vz;
-            }
-            hx_below = hxn;
-            hy_below = hyn;
-            hpar ^= 1;
-        }
+        };
+        // a stage that holds a node of the near-field box or its ring (uniform), else no node asks
+        if (a.nb_w > 0 && cc.x0 <= a.nb_x0 + a.nb_w && cc.x0 + 32 > a.nb_x0 && cc.y0 <= a.nb_y0 + a.nb_w &&
+            cc.y0 + 8 > a.nb_y0 && cc.kb <= a.nb_z0 + a.nb_w && cc.kb + P > a.nb_z0)
+            planes(Flag<true>{});
+        else
+            planes(Flag<false>{});
         acc[0] += (double)(hj * sx + hi * sy + (hi * hj) * sz);
         acc[1] += (double)(hi * mx + hj * my + mz);
-        yee_tma_next(cc, T, P);
+        yee_tma_next(cc, T, P, stride);
         ++it;
+    }
+    if (near_block) {
+        YeeNearShared& sh = *reinterpret_cast<YeeNearShared*>(yee_tma_smem);
+        for (int r = tid; r < (int)(sizeof(YeeNearArgs) / 4); r += 256)
+            reinterpret_cast<unsigned*>(yee_tma_smem)[r] = reinterpret_cast<const unsigned*>(&nr)[r];
+        __syncthreads();
+        yee_near_block<SOLID>(sh, step, acc);
     }
     if (SPLIT && !timed_out) {
         float es = 0.0f, ms = 0.0f;
@@ -441,13 +469,8 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
     }
     __shared__ DevState books;
     unsigned long long was = 0;
-    if (last_block<4>(acc, a.partials, a.nblocks, st, books, was)) {
-        // the last block: with a near-field box it steps the box, adds the box's terms and closes the
-        // books (every other block's cells are in by now: each published its sums after them)
-        if (a.nb_w > 0)
-            yee_near_body<SOLID>(nr, acc, &books);
-        else if (linear_tid() == 0)
-            yee_tma_close(&books, acc, MEDIA, a.g, a.eps_u, a.mu_u, a.volume, a.src_i >= 0);
+    if (last_block<4>(acc, a.partials, gridDim.x, st, books, was)) {
+        if (tid == 0) yee_tma_close(&books, acc, MEDIA, a.g, a.eps_u, a.mu_u, a.volume, a.src_i >= 0 || a.nb_w > 0);
         put_books(st, books, was);
     }
 }
