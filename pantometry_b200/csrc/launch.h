@@ -143,7 +143,7 @@ inline KernelId hall_tma_kernel_id(int shape) {
 bool hall_tma_map(CUtensorMap* map, void* base, int nx, int ny, int nz, unsigned bx, unsigned by, unsigned bz);
 // The FP32 uniform-medium cavity step staged by TMA (padded lattice of row pitch L).
 // `shape` indexes the form's list (kYeeTmaUniformShapes, or kYeeTmaMediaShapes when !a.uniform).
-// `n`: the near-field box the last block steps (n.w = 0 with none; then it is not read).
+// `n`: the near-field box block 0 steps, where a.nb_w is not 0 (else it is not read).
 cudaError_t launch_yee_tma(const YeeStepArgs<float>& a, unsigned L, const YeeMaps& m, int shape, cudaStream_t s,
                            const YeeNearArgs& n = YeeNearArgs{});
 inline size_t yee_tma_smem_bytes(bool media = false, int shape = 0) {

@@ -513,7 +513,7 @@ static __global__ void __launch_bounds__(256, YeeDepth<Real>::min_blocks) yee_st
                 if (fz) { muz = a.mu2[own_h[5]]; cz = a.cch[2][own_h[5]]; }
             }
         }
-        unsigned solid = 0;
+        [[maybe_unused]] unsigned solid = 0;
         if constexpr (SOLID)
             if (compute && in_x && in_y) solid = solid_edges(a.solid, nx, ny, i, j, k);
         const Real hxn = wx - cx * ((S0.ez[ty + 2][tx + 1] - ez0) - (S1.ey[ty + 1][tx + 1] - ey0));

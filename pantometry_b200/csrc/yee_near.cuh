@@ -85,7 +85,7 @@ static_assert(sizeof(YeeNearShared) <= 2 * YeeTmaLayout<3, false>::BYTES, "block
 
 // Run by block 0's 256 threads. Local node indices count from x0 − 1, y0 − 1, z0 − 1: the box is 1 .. W.
 template <bool SOLID>
-__device__ __noinline__ void yee_near_block(YeeNearShared& sh, long long step, double (&acc)[4]) {
+__device__ void yee_near_block(YeeNearShared& sh, long long step, double (&acc)[4]) {
     constexpr int W = YeeNearShared::W, W3 = YeeNearShared::W3, H7 = YeeNearShared::H7, H3 = YeeNearShared::H3,
                   E8 = YeeNearShared::E8, E3 = YeeNearShared::E3, T = 256;
     const YeeNearArgs& a = sh.a;

@@ -341,7 +341,7 @@ static __global__ void __launch_bounds__(256, MINB) yee_tma_step(YeeStepArgs<flo
                     gy = (in_x && by) ? GY[h][ty][tx] : gain0;
                     gz = (in_x && in_y && zin) ? GZ[h][ty][tx] : gain0;
                 }
-                unsigned solid = 0;
+                [[maybe_unused]] unsigned solid = 0;
                 if constexpr (SOLID)
                     if (compute && in_x && in_y) solid = solid_edges(a.solid, nx, ny, i, j, k);
                 YeeHp<float>* hq = hp + hpar;
