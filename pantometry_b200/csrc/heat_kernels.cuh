@@ -430,7 +430,7 @@ __device__ __forceinline__ void heat_plain_books(const HeatPlainArgs& a, double 
 // its own, here and for the wide forms below, since the films' divisions, the slots and the rates
 // cost the others their registers (a Dirichlet 256³ block: 107 µs a step with one kernel for all films,
 // 89 here; the 64³ block's persistent step 5.97 and 5.18).
-template <bool AHEAD>
+template <bool AHEAD, bool FILLED>
 static __global__ void __launch_bounds__(256, PM_HEAT_PLAIN_MIN_BLOCKS) heat_plain_step(HeatPlainArgs a) {
     if (a.st->violated || (AHEAD && heat_refused(a))) return;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -448,6 +448,12 @@ static __global__ void __launch_bounds__(256, PM_HEAT_PLAIN_MIN_BLOCKS) heat_pla
         size_t c = live ? (size_t)i + (size_t)nx * ((size_t)j + (size_t)ny * k0) : 0;
         double below = live && k0 > 0 ? a.told[c - plane] : 0.0;
         double here = live ? a.told[c] : 0.0;
+        const bool xl = i > 0, xh = i + 1 < nx, yl = j > 0, yh = j + 1 < ny;
+        // a filled block's face conductivities: the cell's own low faces, a plane apart in each array, and
+        // the low z face, which is the high one of the plane below
+        const size_t xplane = (size_t)(nx + 1) * ny, yplane = (size_t)nx * (ny + 1);
+        size_t xo = (size_t)i + (size_t)(nx + 1) * j + xplane * k0, yo = (size_t)i + (size_t)nx * j + yplane * k0;
+        [[maybe_unused]] double kzb = FILLED && live ? a.kz[c] : 0.0;
         for (int ka = k0; ka < k1; ka += kFilmPlanes) {
             const int kb = ahead ? min(k1, ka + kFilmPlanes) : k1;
             if (ahead) {
@@ -456,27 +462,42 @@ static __global__ void __launch_bounds__(256, PM_HEAT_PLAIN_MIN_BLOCKS) heat_pla
                 });
                 __syncthreads();
             }
-            for (int k = live ? ka : kb; k < kb; ++k, c += plane) {
-                const double above = k + 1 < nz ? a.told[c + plane] : 0.0;
+            for (int k = live ? ka : kb; k < kb; ++k, c += plane, xo += xplane, yo += yplane) {
                 const double t0 = here;
-                double flux = 0.0;
-                if (a.uniform) {
+                const double above = a.told[k + 1 < nz ? c + plane : c];
+                double flux = 0.0, mob = a.mobility, capc = a.capacity;
+                [[maybe_unused]] double watts = 0.0;
+                [[maybe_unused]] int gap = -1;
+                if constexpr (FILLED) {
+                    // Every load of the plane before the first use of one, a neighbour that is absent read
+                    // at the cell itself and left out of the sum: behind the sum's own branches each pair
+                    // of loads waited for the one before. A radiating block of 150 × 121 × 93 filled cells
+                    // ran 56.5 µs a step so and 48.2 with this; a uniform block has half the loads and ran
+                    // slower (129 × 111 × 101 cells 23.6 and 27.6), so it keeps the branches, in an
+                    // instantiation of its own (21.4).
+                    const double left = a.told[xl ? c - 1 : c], right = a.told[xh ? c + 1 : c];
+                    const double front = a.told[yl ? c - nx : c], back = a.told[yh ? c + nx : c];
+                    // the coefficient arrays hold the outer faces too
+                    const double k0x = a.kx[xo], k1x = a.kx[xo + 1], k0y = a.ky[yo], k1y = a.ky[yo + nx], kza = a.kz[c + plane];
+                    mob = a.mob[c];
+                    capc = a.cap[c];
+                    if (a.src) watts = a.src[c];
+                    if (AHEAD && a.gap_of) gap = a.gap_of[c];
+                    if (xl) flux += k0x * (left - t0);
+                    if (xh) flux += k1x * (right - t0);
+                    if (yl) flux += k0y * (front - t0);
+                    if (yh) flux += k1y * (back - t0);
+                    if (k > 0) flux += kzb * (below - t0);
+                    if (k + 1 < nz) flux += kza * (above - t0);
+                    kzb = kza;
+                } else {
                     const double kf = a.kface;
-                    if (i > 0) flux += kf * (a.told[c - 1] - t0);
-                    if (i + 1 < nx) flux += kf * (a.told[c + 1] - t0);
-                    if (j > 0) flux += kf * (a.told[c - nx] - t0);
-                    if (j + 1 < ny) flux += kf * (a.told[c + nx] - t0);
+                    if (xl) flux += kf * (a.told[c - 1] - t0);
+                    if (xh) flux += kf * (a.told[c + 1] - t0);
+                    if (yl) flux += kf * (a.told[c - nx] - t0);
+                    if (yh) flux += kf * (a.told[c + nx] - t0);
                     if (k > 0) flux += kf * (below - t0);
                     if (k + 1 < nz) flux += kf * (above - t0);
-                } else {
-                    const size_t xr = (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);
-                    const size_t yr = (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);
-                    if (i > 0) flux += a.kx[i + xr] * (a.told[c - 1] - t0);
-                    if (i + 1 < nx) flux += a.kx[i + 1 + xr] * (a.told[c + 1] - t0);
-                    if (j > 0) flux += a.ky[i + yr] * (a.told[c - nx] - t0);
-                    if (j + 1 < ny) flux += a.ky[i + nx + yr] * (a.told[c + nx] - t0);
-                    if (k > 0) flux += a.kz[c] * (below - t0);
-                    if (k + 1 < nz) flux += a.kz[c + plane] * (above - t0);
                 }
                 const bool face = i == 0 || i + 1 == nx || j == 0 || j + 1 == ny || k == 0 || k + 1 == nz;
                 double* const slot = ahead ? heat_film_slot(xf, ft, a, i, j, k - ka) : nullptr;
@@ -484,21 +505,13 @@ static __global__ void __launch_bounds__(256, PM_HEAT_PLAIN_MIN_BLOCKS) heat_pla
                 if (slot) shed = *slot;
                 else if (a.films.exposed && face)
                     shed = AHEAD ? film_flux(a, i, j, k, c, t0) : film_flux_dirichlet(a, i, j, k, t0);
-                const double mob = a.uniform ? a.mobility : a.mob[c];
-                const double capc = a.uniform ? a.capacity : a.cap[c];
                 double nt = t0 + a.dts * mob * (flux - shed);  // add_kelvin, latent <= 0 (solid.rs:1620-1635)
-                if (a.src) {  // solid.rs:1854-1864, after the sweep
-                    const double w = a.src[c];
-                    if (w != 0.0) {
-                        const double joules = w * a.dts;
-                        nt += joules / capc;
-                        acc[2] += joules;
-                    }
+                if (FILLED && watts != 0.0) {  // solid.rs:1854-1864, after the sweep
+                    const double joules = watts * a.dts;
+                    nt += joules / capc;
+                    acc[2] += joules;
                 }
-                if (AHEAD && a.gap_of) {
-                    const int g = a.gap_of[c];
-                    if (g >= 0) nt = heat_gap_cell(a, g, t0, capc, nt, rate);
-                }
+                if (FILLED && AHEAD && gap >= 0) nt = heat_gap_cell(a, gap, t0, capc, nt, rate);
                 a.tnew[c] = nt;
                 acc[0] += capc * (nt - a.reference);                  // solid.rs:1583-1590
                 if (shed != 0.0) acc[1] += a.dts * mob * shed * capc;  // solid.rs:1821-1823
@@ -867,6 +880,10 @@ static __global__ void __launch_bounds__(256, RAD ? 4 : 1) heat_f32_step(HeatF32
         const bool xl = i > 0, xh = i + 1 < nx, yl = j > 0, yh = j + 1 < ny;
         const bool edge_xy = !(xl && xh && yl && yh);
         double col_shed = 0.0;
+        // a filled block's face conductivities, as in heat_plain_step
+        const size_t xplane = (size_t)(nx + 1) * ny, yplane = (size_t)nx * (ny + 1);
+        size_t xo = (size_t)i + (size_t)(nx + 1) * j + xplane * k0, yo = (size_t)i + (size_t)nx * j + yplane * k0;
+        [[maybe_unused]] float kzb = FILLED && live ? __ldg(a.kz + c) : 0.0f;
         for (int ka = k0; ka < k1; ka += kFilmPlanes) {
             const int kb = ahead ? min(k1, ka + kFilmPlanes) : k1;
             if (ahead) {
@@ -875,19 +892,29 @@ static __global__ void __launch_bounds__(256, RAD ? 4 : 1) heat_f32_step(HeatF32
                 });
                 __syncthreads();
             }
-            for (int k = live ? ka : kb; k < kb; ++k, c += plane) {
-                const float above = (k + 1 < nz) ? __ldg(a.dold + c + plane) : 0.0f;
+            for (int k = live ? ka : kb; k < kb; ++k, c += plane, xo += xplane, yo += yplane) {
+                const float above = __ldg(a.dold + (k + 1 < nz ? c + plane : c));
+                [[maybe_unused]] float mc = 0.0f;
+                [[maybe_unused]] double capc = 0.0, watts = 0.0;
                 float s = 0.0f;
                 if constexpr (FILLED) {
-                    // solid.rs:1773-1826 in the reference's arm order, each face's own conductivity
-                    const size_t xr = (size_t)(nx + 1) * ((size_t)j + (size_t)ny * k);
-                    const size_t yr = (size_t)nx * ((size_t)j + (size_t)(ny + 1) * k);
-                    if (xl) s += __ldg(a.kx + i + xr) * (__ldg(a.dold + c - 1) - here);
-                    if (xh) s += __ldg(a.kx + i + 1 + xr) * (__ldg(a.dold + c + 1) - here);
-                    if (yl) s += __ldg(a.ky + i + yr) * (__ldg(a.dold + c - nx) - here);
-                    if (yh) s += __ldg(a.ky + i + nx + yr) * (__ldg(a.dold + c + nx) - here);
-                    if (k > 0) s += __ldg(a.kz + c) * (below - here);
-                    if (k + 1 < nz) s += __ldg(a.kz + c + plane) * (above - here);
+                    // solid.rs:1773-1826 in the reference's arm order, each face's own conductivity; every load
+                    // of the plane before the first use of one, as in heat_plain_step (110 × 111 × 101 cells
+                    // 16.5 µs a step before and 14.3 with this)
+                    const float left = __ldg(a.dold + (xl ? c - 1 : c)), right = __ldg(a.dold + (xh ? c + 1 : c));
+                    const float front = __ldg(a.dold + (yl ? c - nx : c)), back = __ldg(a.dold + (yh ? c + nx : c));
+                    const float k0x = __ldg(a.kx + xo), k1x = __ldg(a.kx + xo + 1), k0y = __ldg(a.ky + yo),
+                                k1y = __ldg(a.ky + yo + nx), kza = __ldg(a.kz + c + plane);
+                    mc = __ldg(a.m + c);
+                    capc = __ldg(a.cap + c);
+                    if (a.src) watts = __ldg(a.src + c);
+                    if (xl) s += k0x * (left - here);
+                    if (xh) s += k1x * (right - here);
+                    if (yl) s += k0y * (front - here);
+                    if (yh) s += k1y * (back - here);
+                    if (k > 0) s += kzb * (below - here);
+                    if (k + 1 < nz) s += kza * (above - here);
+                    kzb = kza;
                 } else {
                     if (xl) s += __ldg(a.dold + c - 1) - here;
                     if (xh) s += __ldg(a.dold + c + 1) - here;
@@ -926,16 +953,11 @@ static __global__ void __launch_bounds__(256, RAD ? 4 : 1) heat_f32_step(HeatF32
                 float nd;
                 if constexpr (FILLED) {
                     // add_kelvin (solid.rs:1620-1635); stored heat C·dev and shed heat C·dt·mob·shed
-                    const float mc = __ldg(a.m + c);
                     nd = here + mc * (s - shed);
-                    const double capc = __ldg(a.cap + c);
-                    if (a.src) {  // solid.rs:1854-1864, after the sweep: the joules in FP64, the rise in f32
-                        const double w = __ldg(a.src + c);
-                        if (w != 0.0) {
-                            const double joules = w * a.dts;
-                            nd += (float)(joules / capc);
-                            acc[FILLED ? 2 : 0] += joules;
-                        }
+                    if (watts != 0.0) {  // solid.rs:1854-1864, after the sweep: the joules in FP64, the rise in f32
+                        const double joules = watts * a.dts;
+                        nd += (float)(joules / capc);
+                        acc[FILLED ? 2 : 0] += joules;
                     }
                     acc[0] += capc * (double)nd;
                     if (shed != 0.0f) acc[1] += capc * (double)(mc * shed);

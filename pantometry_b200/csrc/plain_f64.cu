@@ -8,9 +8,10 @@ namespace pm {
 
 cudaError_t launch_heat_plain(const HeatPlainArgs& a, cudaStream_t s) {
     const bool ahead = a.films.ahead != 0;
-    auto k = a.quads   ? (ahead ? heat_plain_quad_step<true> : heat_plain_quad_step<false>)
-             : a.pairs ? (ahead ? heat_plain_pair_step<true> : heat_plain_pair_step<false>)
-                       : (ahead ? heat_plain_step<true> : heat_plain_step<false>);
+    auto k = a.quads     ? (ahead ? heat_plain_quad_step<true> : heat_plain_quad_step<false>)
+             : a.pairs   ? (ahead ? heat_plain_pair_step<true> : heat_plain_pair_step<false>)
+             : a.uniform ? (ahead ? heat_plain_step<true, false> : heat_plain_step<false, false>)
+                         : (ahead ? heat_plain_step<true, true> : heat_plain_step<false, true>);
     k<<<a.nblocks, tile_block(), 0, s>>>(a);
     return cudaGetLastError();
 }
@@ -229,7 +230,7 @@ int occupancy_f64(KernelId id) {
     int n = 0;
     cudaError_t e = cudaSuccess;
     switch (id) {
-        case kHeatPlain: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_step<true>, 256, 0); break;
+        case kHeatPlain: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_step<true, true>, 256, 0); break;
         case kHeatPlainPair: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_step<true>, 256, 0); break;
         case kHeatPlainQuad: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_quad_step<true>, 256, 0); break;
         case kHeatPlainSteps: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<8, true>, 256, 0); break;
