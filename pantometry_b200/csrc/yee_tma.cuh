@@ -7,8 +7,8 @@
 // the ε the update itself used.
 //
 // Layout. The handle keeps all six components on the (nx+1) × (ny+1) × (nz+1) node lattice with
-// one index n = i + L·(j + (ny+1)·k), L = nx+1 rounded up to a multiple of 4 (so every row pitch
-// is a multiple of 16 bytes, as TMA requires). A component's lattice positions outside its own
+// one index n = i + L·(j + (ny+1)·k), L = nx+1 rounded up to a multiple of 8 (every row starts on a
+// 32-byte sector; TMA asks for 16 bytes, pm_cavity_create says what the rest is for). A component's lattice positions outside its own
 // extent (cavity.rs:112-123) are padding: zero, never written.
 //
 // Walk. Tiles are 32 × 8 columns of the lattice over a z-chunk, taken by a persistent grid in
