@@ -853,7 +853,7 @@ def cavity_record(local, stream, peak, n=384, timed_steps=2000, compare_steps=10
                       "roofline_frac": round(96 * cells / (ms64 / timed_steps * 1e-3) / 1e9 / peak, 4)},
         "fp32_over_f64": round(value / plain, 3),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "kernel": "yee_tma_step + yee_near_step (FP32)",
+                     "frac": round(achieved / peak, 4), "kernel": "yee_tma_step (FP32)",
                      "bytes_per_timestep": 48 * cells,
                      "traffic": round(YEE_F32_TRAFFIC_PER_CELL * cells), "traffic_source": "ncu capture at 256^3, scaled by cells"},
         "error_vs_f64": {"ledger_rel": worst, "at_timestep": at, "final_ledger_rel": final,
