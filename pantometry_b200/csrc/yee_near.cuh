@@ -175,7 +175,9 @@ __device__ void yee_near_block(YeeNearShared& sh, long long step, double (&acc)[
             if (q == 2 && gi == a.src_i && gj == a.src_j && gk == a.src_k) {
                 // soft current: ε dE/dt = ∇×H − J, with the σ term's semi-implicit divisor
                 const double e = a.eps_src, ss = a.sig_src;
-                v = v - (a.dt / e) / (1.0 + (ss * a.dt / (2.0 * e))) * jsrc;
+                // (the product rounded by itself: near its zeros ez is all cancellation, and one rounding
+                // here moved its last bits, which thousands of f32 steps then carry through the box)
+                v = v - __dmul_rn((a.dt / e) / (1.0 + (ss * a.dt / (2.0 * e))), jsrc);
                 acc[3] += -(a.dt * a.volume) * jsrc * (0.5 * (e0 + v));
             }
             v = interior ? v : 0.0;
