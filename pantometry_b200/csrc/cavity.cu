@@ -390,14 +390,16 @@ struct Cavity : Handle {
     // history, and only then zeroes the obstacles' edges (cavity.rs:1497-1499, 1159-1163). The
     // step kernels then leave those edges alone, the walls run, E is copied to `stale` (the history
     // lives there from then on) and yee_enforce_solid zeroes the edges.
-    // Obstacles whose edges stay off such a wall and off the plane inside it are out of the walls'
-    // reach and out of their history, so the step kernels zero them as they do in a conducting box.
+    // A wall's update and history read its own plane and the plane inside it. Obstacles whose edges stay
+    // off those of all six walls are out of reach, so the step kernels zero them as they do in a conducting
+    // box. A conducting wall counts too: it may be set open after these steps, and its first update then
+    // reads the history that they left.
     int solid_lo[3] = {0, 0, 0}, solid_hi[3] = {0, 0, 0};  // the solid cells' least and greatest indices
     bool solid_after_walls() const {
-        if (!any_solid) return false;
+        if (!any_solid || !open_or_magnetic()) return false;
         const int n[3] = {nx, ny, nz};
         for (int a = 0; a < 3; ++a)
-            if ((boundary[2 * a] != 0 && solid_lo[a] <= 1) || (boundary[2 * a + 1] != 0 && solid_hi[a] >= n[a] - 2)) return true;
+            if (solid_lo[a] <= 1 || solid_hi[a] >= n[a] - 2) return true;
         return false;
     }
     pm_status ensure_stale() {
