@@ -107,7 +107,10 @@ static __global__ void __launch_bounds__(256) room_step(RoomArgs<Real> a) {
 // The books stay off that path, as in the many-step heat kernels: each warp leaves its sum of step s in
 // block 0, whose last warp (it takes no nodes) reduces and audits it while the others run step s + 1. A
 // failed audit is told to every block before step s + 1's barrier, and the call ends with step s's
-// state: p holds three steps, so s and s − 1 are intact, and vx and vy two.
+// state: p holds three steps, so s and s − 1 are intact, and vx and vy two. The word that tells it goes by
+// the step's parity: a thread reads step s's word after barrier s and before barrier s + 1, and that word is
+// not written again before step s + 2, so every thread of the cluster leaves at the same barrier. (One word
+// for all steps could be set for step s + 1 before a late thread had read it for step s.)
 constexpr int kRoomThreads = 512;  // nodes are taken by these; one warp more keeps the books
 constexpr int kRoomMaxCluster = 16;
 constexpr int kRoomChunk = 4096;  // steps a launch
@@ -136,7 +139,7 @@ static __global__ void __launch_bounds__(kRoomThreads + 32, 1) room_steps(RoomSt
     extern __shared__ __align__(16) unsigned char room_smem[];
     __shared__ double part[2][kRoomMaxCluster * WARPS];  // block 0's: each warp's sum of a step, by its parity
     __shared__ DevState books;                           // block 0's
-    __shared__ int stop;
+    __shared__ int stop[2];                              // by the parity of the step whose barrier they end
     if (a.st->violated) return;  // every block reads the same word
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
@@ -154,7 +157,7 @@ static __global__ void __launch_bounds__(kRoomThreads + 32, 1) room_steps(RoomSt
         if (j >= 0 && j < ny - 1 && j < r1) VY[l] = a.vy[0][i + (size_t)nx * j];
         if (j >= r0 && j < r1 && i < nx - 1) VX[l - nx] = a.vx[0][i + (size_t)(nx - 1) * j];
     }
-    if (tid == 0) stop = 0;
+    if (tid == 0) stop[0] = stop[1] = 0;
     if (keeper && lane == 0) books = *a.st;
     Real* const below_p = rank > 0 ? cluster.map_shared_rank(P, rank - 1) : nullptr;
     Real* const above_p = rank + 1 < blocks ? cluster.map_shared_rank(P, rank + 1) : nullptr;
@@ -224,10 +227,10 @@ static __global__ void __launch_bounds__(kRoomThreads + 32, 1) room_steps(RoomSt
             warp_sum<1>(acc);
             if (lane == 0) sums[(s & 1) * (kRoomMaxCluster * WARPS) + warp] = acc[0];
         } else if (keeper && s > 0 && audit(s - 1)) {
-            if (lane < blocks) *cluster.map_shared_rank(&stop, lane) = 1;
+            if (lane < blocks) *cluster.map_shared_rank(&stop[s & 1], lane) = 1;
         }
         cluster.sync();
-        if (stop) {  // step s − 1 failed its audit: the state it left is the present slot's
+        if (stop[s & 1]) {  // step s − 1 failed its audit: the state it left is the present slot's
             failed = true;
             done = s;
             break;
