@@ -434,6 +434,7 @@ struct Cavity : Handle {
             a.ry[q] = tma ? (unsigned)(ny + 1) : (unsigned)ey;
         }
         a.nx = nx; a.ny = ny; a.nz = nz;
+        for (int w = 0; w < 6; ++w) a.conducting |= boundary[w] == 0 ? 1 << w : 0;
         return a;
     }
     // After the walls of the step from `par`: E (before the obstacles are zeroed) becomes Mur's
@@ -452,25 +453,31 @@ struct Cavity : Handle {
         const double c_dt = wave_speed() * dt;
         a.k = (Real)((c_dt - dx) / (c_dt + dx));  // cavity.rs:1075-1078
         const int n[3] = {nx, ny, nz};
-        auto launch = [&](auto&& ours) {  // the walls `ours` names, in one launch
+        auto launch = [&](auto&& kind_of) {  // the walls `kind_of` gives a kind, in one launch
             a.first[0] = 0;
             for (int w = 0; w < 6; ++w) {
-                a.kind[w] = !ours(w) ? 0 : boundary[w] == 1 ? 1 : prev ? 2 : 3;
+                a.kind[w] = kind_of(w);
                 const unsigned u = (unsigned)n[w < 2 ? 1 : 0], v = (unsigned)n[w < 4 ? 2 : 1];
                 a.first[w + 1] = a.first[w] + (a.kind[w] ? u * (v + 1) + (u + 1) * v : 0);
             }
             return launch_yee_walls<Real>(a, s);
         };
-        // an axis of one cell: its walls' inner neighbours lie on the opposite wall, so one wall at a
-        // time, in the reference's order (magnetic walls, then open ones)
+        auto kind = [&](int w) { return boundary[w] == 0 ? 0 : boundary[w] == 1 ? 1 : prev ? 2 : 3; };
         bool thin = false;
         for (int w = 0; w < 6; ++w) thin = thin || (boundary[w] != 0 && n[w >> 1] < 2);
-        if (!thin) return launch([&](int w) { return boundary[w] != 0; });
-        for (int kind : {1, 2})
+        if (!thin) return launch(kind);
+        // An axis of one cell: its walls' inner neighbours lie on the opposite wall. The update reaches no
+        // edge of a wall (cavity.rs:1383-1452), so those edges take back the last step's E, which the step
+        // kernel wrote over with the conducting walls' zero; then one wall at a time, in the reference's
+        // order (magnetic walls, then open ones).
+        for (int q = 0; q < 3; ++q) a.pe[q] = f[par][q].as<Real>();
+        cudaError_t e = launch([&](int w) { return boundary[w] != 0 && n[w >> 1] < 2 ? 4 : 0; });
+        if (e != cudaSuccess) return e;
+        for (int q = 0; q < 3; ++q) a.pe[q] = stale_history ? stale[q].as<Real>() : f[par][q].as<Real>();
+        for (int b : {1, 2})
             for (int w = 0; w < 6; ++w) {
-                if (boundary[w] != kind) continue;
-                cudaError_t e = launch([&](int one) { return one == w; });
-                if (e != cudaSuccess) return e;
+                if (boundary[w] != b) continue;
+                if ((e = launch([&](int one) { return one == w ? kind(w) : 0; })) != cudaSuccess) return e;
             }
         return cudaSuccess;
     }

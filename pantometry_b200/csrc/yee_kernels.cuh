@@ -665,9 +665,11 @@ struct YeeWallArgs {
     int nx, ny, nz;
     unsigned rx[3], ry[3];
     // Per wall 0..5 (XLow, XHigh, YLow, YHigh, ZLow, ZHigh): 0 not this launch's, 1 mirror (magnetic),
-    // 2 Mur (open), 3 zero (open, no history yet); and the first of each wall's edges among the launch's
+    // 2 Mur (open), 3 zero (open, no history yet), 4 take back pe (an axis of one cell, before its walls
+    // are applied); and the first of each wall's edges among the launch's
     int kind[6];
     unsigned first[7];
+    int conducting;     // bit w: wall w conducts, and holds the edges it shares with others at zero
     Real k;             // Mur's coefficient (cΔt − Δ)/(cΔt + Δ)
 };
 
@@ -711,7 +713,8 @@ __device__ __forceinline__ Real yee_wall_value(int kind, Real k, Real inner, Rea
 // inner neighbour; where two walls meet, that neighbour lies on the earlier one, and its value then is
 // formed here by that wall's own rule from its inner neighbour, which no wall touches. So every edge
 // comes from edges off the walls and the history alone, whatever order the threads run in. (An axis of one
-// cell has its two walls one edge apart: the host then launches one wall at a time.) Six launches, one a
+// cell has its two walls one edge apart: the host then gives its edges back the last step's E and launches
+// one wall at a time.) Six launches, one a
 // wall, with E copied aside and the obstacle zeroed after them, were half of an open box's step: 101 × 83 ×
 // 67 cells around an obstacle in f64 ran 64.8 µs a step with them and 31.0 with this, 32 × 24 × 24 in FP32
 // 40.0 and 19.4.
@@ -738,12 +741,17 @@ static __global__ void yee_walls(YeeWallArgs<Real> a) {
         const int w2 = at[other] == 0 ? 2 * other : at[other] == n[other] ? 2 * other + 1 : -1;
         const int rank2 = w2 < 0 ? -1 : yee_wall_rank(a, w2);
         if (rank2 > yee_wall_rank(a, w)) continue;  // the other wall is the last: its thread's edge
+        if (a.kind[w] == 4 && w2 >= 0 && ((a.conducting >> w2) & 1)) continue;
         auto index = [&](const int(&x)[3]) {
             return (size_t)x[0] + (size_t)a.rx[q] * ((size_t)x[1] + (size_t)a.ry[q] * (size_t)x[2]);
         };
         Real* const e = a.e[q];
         const Real* const pe = a.pe[q];
         const size_t ai = index(at);
+        if (a.kind[w] == 4) {
+            e[ai] = pe[ai];
+            continue;
+        }
         at[axis] = (w & 1) ? n[axis] - 1 : 1;
         const size_t bi = index(at);
         Real inner;
