@@ -495,7 +495,6 @@ struct Cavity : Handle {
             if (near_on()) {
                 // the box's terms and the source are those of the grid's block 0, which takes no tiles
                 const YeeNearArgs n = nargs(par, h, t);
-                t.nblocks = std::max(1u, std::min(t.nblocks, wave_of(yee_tma_kernel_id(!uniform, yshape)) - 1));
                 t.nb_x0 = near_x0; t.nb_y0 = near_y0; t.nb_z0 = near_z0; t.nb_w = near_w;
                 t.src_i = t.src_j = t.src_k = -1;
                 e = launch_yee_tma(t, L, maps[par], yshape, s, n);
@@ -697,7 +696,7 @@ struct Cavity : Handle {
     // P·m − 1 planes, so a chunk and the plane below it fill whole stages).
     YeeStepArgs<float> targs(int par, double dt) const {
         YeeStepArgs<float> a = sargs<float>(par, dt);
-        const unsigned w = wave_of(yee_tma_kernel_id(!uniform, yshape));
+        const unsigned w = yee_tile_blocks(wave_of(yee_tma_kernel_id(!uniform, yshape)), near_on());
         const int P = yee_tma_shape(!uniform, yshape).planes;
         // the wall pass takes the last column and row when the tiles then cover the rest exactly;
         // a source on one of those edges stays with the tiles, which book its work

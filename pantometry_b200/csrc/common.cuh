@@ -13,29 +13,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tiles.h"
+
 namespace pm {
-
-// The tiling every step kernel walks: 32 × 8 columns of cells (one warp row per y), each
-// marched through `zc` planes by its thread. A persistent grid of blocks takes tiles
-// blockIdx.x, blockIdx.x + gridDim.x, ... in that fixed order, so every thread's share of a
-// reduction is summed in the same order on every run.
-struct Tiles {
-    int nx, ny, nz, zc;
-    int ntx, nty, ntz;
-    long long ntiles;
-    int rows;  // rows of a tile: the block's y extent (8 but in the many-step heat kernels)
-};
-
-__host__ __device__ inline Tiles make_tiles(int nx, int ny, int nz, int zc, int rows = 8) {
-    Tiles t;
-    t.nx = nx; t.ny = ny; t.nz = nz; t.zc = zc;
-    t.rows = rows;
-    t.ntx = (nx + 31) / 32;
-    t.nty = (ny + rows - 1) / rows;
-    t.ntz = (nz + zc - 1) / zc;
-    t.ntiles = (long long)t.ntx * t.nty * t.ntz;
-    return t;
-}
 
 // A compile-time flag as an argument.
 template <bool B>

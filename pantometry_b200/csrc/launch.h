@@ -25,28 +25,6 @@ inline dim3 tile_block() { return dim3(32, 8, 1); }
 constexpr int kBlocksPerSM = 8;
 constexpr int kMeasureBlocks = 592;  // 4 × 148 SMs, for the flat element-wise kernels
 
-// The z-chunk of a z-marching kernel, a multiple of the `lo` planes it takes at a time less `off`. A
-// block takes ceil(tiles / wave) tiles one after another, and a tile costs its planes and about one more
-// (the planes below and above its first and last): the chunk with the least of that product is taken,
-// with a quarter of a tile for the uneven end. Large grids keep chunks of 6 to 20 planes; a grid that
-// does not fill the SMs takes the thinnest, since a step is then as long as one tile. Measured,
-// µs a step, chunks of 4, 8, 16 or 32 planes by their even spread alone and by this rule: a radiating f64
-// block of 150 × 121 × 93 cells 67.6 and 55.8, a filled f64 32³ one 9.9 and 6.4, a lossy f64 32 × 24 × 31
-// cavity 11.3 and 9.5, an FP32 31 × 27 × 43 one 17.2 and 15.6; a 256³ FP32 hall 96.4 and 96.4.
-inline int choose_zc(int nx, int ny, int nz, unsigned resident, int lo = 1, int off = 0) {
-    int best = lo - off;
-    double best_cost = -1.0;
-    for (int zc = lo - off; zc < nz + lo && zc <= 64; zc += lo) {
-        const long long rounds = (make_tiles(nx, ny, nz, zc).ntiles + resident - 1) / resident;
-        const double cost = ((double)rounds + 0.25) * (zc + 1);
-        if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = zc; }
-    }
-    return best;
-}
-inline unsigned grid_for(const Tiles& t, unsigned resident) {
-    return (unsigned)(t.ntiles < (long long)resident ? t.ntiles : (long long)resident);
-}
-
 // Opt `kernel` in to `bytes` of dynamic shared memory on the current device. The attribute
 // belongs to the function on one device, so the opt-in is recorded per (kernel, device) and made
 // once for each, under a lock (handles on several devices and several host threads share it).

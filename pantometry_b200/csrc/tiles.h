@@ -1,0 +1,58 @@
+// How a grid is cut into tiles for the z-marching kernels, and the blocks that take them. Host code that a
+// plain C++ compiler takes too.
+#pragma once
+
+namespace pm {
+
+// The tiling every step kernel walks: 32 × 8 columns of cells (one warp row per y), each
+// marched through `zc` planes by its thread. A persistent grid of blocks takes tiles
+// blockIdx.x, blockIdx.x + gridDim.x, ... in that fixed order, so every thread's share of a
+// reduction is summed in the same order on every run.
+struct Tiles {
+    int nx, ny, nz, zc;
+    int ntx, nty, ntz;
+    long long ntiles;
+    int rows;  // rows of a tile: the block's y extent (8 but in the many-step heat kernels)
+};
+
+inline Tiles make_tiles(int nx, int ny, int nz, int zc, int rows = 8) {
+    Tiles t;
+    t.nx = nx; t.ny = ny; t.nz = nz; t.zc = zc;
+    t.rows = rows;
+    t.ntx = (nx + 31) / 32;
+    t.nty = (ny + rows - 1) / rows;
+    t.ntz = (nz + zc - 1) / zc;
+    t.ntiles = (long long)t.ntx * t.nty * t.ntz;
+    return t;
+}
+
+// The z-chunk of a z-marching kernel, a multiple of the `lo` planes it takes at a time less `off`. A
+// block takes ceil(tiles / wave) tiles one after another, and a tile costs its planes and about one more
+// (the planes below and above its first and last): the chunk with the least of that product is taken,
+// with a quarter of a tile for the uneven end. Large grids keep chunks of 6 to 20 planes; a grid that
+// does not fill the SMs takes the thinnest, since a step is then as long as one tile. Measured,
+// µs a step, chunks of 4, 8, 16 or 32 planes by their even spread alone and by this rule: a radiating f64
+// block of 150 × 121 × 93 cells 67.6 and 55.8, a filled f64 32³ one 9.9 and 6.4, a lossy f64 32 × 24 × 31
+// cavity 11.3 and 9.5, an FP32 31 × 27 × 43 one 17.2 and 15.6; a 256³ FP32 hall 96.4 and 96.4.
+inline int choose_zc(int nx, int ny, int nz, unsigned resident, int lo = 1, int off = 0) {
+    int best = lo - off;
+    double best_cost = -1.0;
+    for (int zc = lo - off; zc < nz + lo && zc <= 64; zc += lo) {
+        const long long rounds = (make_tiles(nx, ny, nz, zc).ntiles + resident - 1) / resident;
+        const double cost = ((double)rounds + 0.25) * (zc + 1);
+        if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = zc; }
+    }
+    return best;
+}
+// The blocks of a wave of yee_tma_step that take tiles: with a near-field box one is the box's. Tiles cut for
+// the whole wave and stepped by one block less took a round more wherever they filled their rounds, a cavity
+// in a hundred. Those, µs a step for the whole wave and for the blocks there are: 64 × 64 × 256 of mixed ε
+// 24.9 and 21.0, 192 × 32 × 256 32.4 and 30.0, 217 × 145 × 255 of one medium 89.6 and 81.9; the smallest,
+// whose last round is a few tiles long, lose as they leave their thin chunks: 59 × 46 × 146 13.5 and 14.4,
+// 64 × 32 × 256 of mixed ε 17.1 and 18.2.
+inline unsigned yee_tile_blocks(unsigned wave, bool near) { return near && wave > 1 ? wave - 1 : wave; }
+inline unsigned grid_for(const Tiles& t, unsigned resident) {
+    return (unsigned)(t.ntiles < (long long)resident ? t.ntiles : (long long)resident);
+}
+
+}  // namespace pm
