@@ -365,30 +365,42 @@ static __global__ void __launch_bounds__(kEnsConsumers + 32, PM_ENS_TMA_MIN_BLOC
     }
 }
 
-// The books of every block after ens_tma_step: a thread block per block of the ensemble sums its bricks'
-// partials in a fixed order (thread-strided, then the block's tree), then runs its ledger and audit. A
-// block held at the step's start (violated) was copied, not stepped, and is left alone. A 128³ block
-// has 512 bricks of 8 warps' partials, and one warp summing them sat on 128 dependent round trips: a
-// step of 160 blocks of 16 to 128 cells an axis ran 170.2 µs with a warp per block, 166.2 with this, a
-// step of 20 blocks of 100 to 128 cells 79.2 and 75.1.
+// The books of every block after ens_tma_step: T threads per block of the ensemble sum its bricks'
+// partials in a fixed order (thread-strided, then the threads' tree), then run its ledger and audit. A
+// block held at the step's start (violated) was copied, not stepped, and is left alone.
+// A 128³ block has 512 bricks of 8 warps' partials, and one warp summing them sits on 128 dependent round
+// trips; small blocks have a few dozen partials, and a thread block for each is mostly idle threads to
+// launch. So a warp sums where no block of the ensemble has more than kEnsWarpBricks bricks. Measured, µs
+// a step, a warp and a thread block per block (largest block's bricks): 16384 blocks of 16³ (2) 328 and
+// 363, 4096 of 16 to 24 cells an axis (6) 167 and 175, 2000 of 16 to 32 (8) 118.6 and 120.8; 512 of 32 to 40
+// (30) 109.8 and 107.4, 160 of 16 to 128 (512) 158.9 and 144.5, 20 of 100 to 128 (512) 88.2 and 73.9.
+constexpr unsigned kEnsWarpBricks = 16;
+template <int T>
 static __global__ void __launch_bounds__(256) ens_tma_books(const EnsArgs<float> a) {
-    const unsigned gi = blockIdx.x;
+    static_assert(T == 32 || T == 256, "a warp or a thread block");
+    const unsigned gi = T == 256 ? blockIdx.x : blockIdx.x * (256 / T) + threadIdx.x / T;
+    if (gi >= a.ngrids) return;  // a whole warp
+    const unsigned lane = T == 256 ? threadIdx.x : threadIdx.x % T;
     DevState* st = a.states + gi;
-    __shared__ double red[32 * 2];
-    __shared__ int held;
-    if (threadIdx.x == 0) held = st->violated;
+    int held = 0;
+    if (lane == 0) held = st->violated;
     const EnsGrid& g = a.grids[gi];
     double v[2] = {0.0, 0.0};
     const double2* part = reinterpret_cast<const double2*>(a.partials) + (size_t)g.first_brick * 8;
     const unsigned count = g.nbricks * 8;
 #pragma unroll 4
-    for (unsigned q = threadIdx.x; q < count; q += 256) {
+    for (unsigned q = lane; q < count; q += T) {
         const double2 p = part[q];
         v[0] += p.x;
         v[1] += p.y;
     }
-    block_sum<2>(v, red);
-    if (threadIdx.x == 0 && !held) {
+    if constexpr (T == 256) {
+        __shared__ double red[32 * 2];
+        block_sum<2>(v, red);
+    } else {
+        warp_sum<2>(v);
+    }
+    if (lane == 0 && !held) {
         const double stored = g.capacity * v[0];
         st->lost += g.capacity * v[1];
         double total = 0.0, scale = 0.0;

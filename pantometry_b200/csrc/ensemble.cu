@@ -155,6 +155,7 @@ struct Ensemble : Handle {
     std::vector<CUtensorMap> maps;
     DBuf dmaps, dinfos;
     DBuf dwork;  // the TMA walk's two counters (next brick, CTAs done), zero between launches
+    bool wide_books = false;  // the TMA step's books: a thread block per block of the ensemble, else a warp
     int shape = 0;
     long long generation = 0;  // bumped when the brick list changes (the graph cache key)
     DBuf field[2], stage, dgrids, dbricks, dstates, bpartials, saved, saved_states;
@@ -172,6 +173,7 @@ struct Ensemble : Handle {
             return fail(PM_BAD_ARG, s.cells == 4 ? "quad brick shapes are f32 only" : "pair brick shapes are f64 only");
         const int bx = s.x(), by = s.y();
         bricks.clear();
+        unsigned most = 0;  // bricks of one block
         for (size_t g = 0; g < grids.size(); ++g) {
             EnsGrid& e = grids[g];
             e.first_brick = (unsigned)bricks.size();
@@ -187,7 +189,9 @@ struct Ensemble : Handle {
                         bricks.push_back(b);
                     }
             e.nbricks = (unsigned)bricks.size() - e.first_brick;
+            most = std::max(most, e.nbricks);
         }
+        wide_books = most > kEnsWarpBricks;
         if (bricks.size() >= (size_t)UINT32_MAX) return fail(PM_BAD_ARG, "too many bricks");
         if (tma) {  // the per-brick records the TMA kernel copies with each stage
             std::vector<EnsBrickInfo> infos(bricks.size());
@@ -250,7 +254,7 @@ struct Ensemble : Handle {
             t.infos = dinfos.as<EnsBrickInfo>();
             t.work = dwork.as<unsigned>();
             const unsigned w = wave_of(kEnsTma);
-            return launch_ens_tma(t, std::min<unsigned>(w, (unsigned)std::max<size_t>(bricks.size(), 1)), s);
+            return launch_ens_tma(t, std::min<unsigned>(w, (unsigned)std::max<size_t>(bricks.size(), 1)), wide_books, s);
         }
         return launch_ens<float>(args<float>(par), measure, nblocks(), s);
     }

@@ -189,11 +189,12 @@ cudaError_t launch_yee_relayout(const void* src, bool src_f64, void* dst, bool d
     return cudaGetLastError();
 }
 
-cudaError_t launch_ens_tma(const EnsTmaArgs& t, unsigned nblocks, cudaStream_t s) {
+cudaError_t launch_ens_tma(const EnsTmaArgs& t, unsigned nblocks, bool wide_books, cudaStream_t s) {
     const int smem = (int)ens_tma_smem_bytes();
     cudaError_t e = launch_smem(ens_tma_step<kEnsTmaPlanes, kEnsTmaStages>, nblocks, kEnsConsumers + 32, smem, s, t);
     if (e != cudaSuccess) return e;
-    ens_tma_books<<<t.e.ngrids, 256, 0, s>>>(t.e);
+    if (wide_books) ens_tma_books<256><<<t.e.ngrids, 256, 0, s>>>(t.e);
+    else ens_tma_books<32><<<(t.e.ngrids + 7) / 8, 256, 0, s>>>(t.e);
     return cudaGetLastError();
 }
 

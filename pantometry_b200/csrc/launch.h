@@ -140,8 +140,9 @@ cudaError_t launch_yee_near_seed(const YeeNearArgs& a, cudaStream_t s);
 // src_f64 / dst_f64 select double or float for each side.
 cudaError_t launch_yee_relayout(const void* src, bool src_f64, void* dst, bool dst_f64, int ex, int ey, int ez,
                                 unsigned L, unsigned ny1, int to_padded, cudaStream_t s);
-// One FP32 ensemble step over 32 × 8-column bricks, staged by TMA.
-cudaError_t launch_ens_tma(const EnsTmaArgs& t, unsigned nblocks, cudaStream_t s);
+// One FP32 ensemble step over 32 × 8-column bricks, staged by TMA, and its books (wide_books: a thread block
+// per block of the ensemble, else a warp).
+cudaError_t launch_ens_tma(const EnsTmaArgs& t, unsigned nblocks, bool wide_books, cudaStream_t s);
 // One block between kelvin on the host's layout and f32 deviations on padded rows.
 cudaError_t launch_ens_relayout(const double* kelvin, float* dev, double* out, int nx, int ny, int nz, int pitch,
                                 double t0, int to_dev, cudaStream_t s);
