@@ -568,10 +568,17 @@ __device__ __forceinline__ double heat_ld(const double* p) {
 // One tile of the wide form for one step, from `told` into `tnew`: W adjacent cells of a row per
 // thread (W = 2, the pair form, or 4), the arithmetic the one-step kernels and the persistent
 // many-step kernel run, so they agree bit for bit. Each row of W cells comes in 16-byte loads.
-template <bool CG, int W, int ROWS, bool AHEAD>
+// FILMS: which films the block has and where they are formed, an instantiation each (see heat_plain_step).
+enum HeatFilmsAt : int {
+    kFilmsDirichlet,  // none, or Dirichlet ones: in the march
+    kFilmsMarch,      // any that do not radiate: in the march (the many-step kernel)
+    kFilmsAhead,      // any: those of x and y face cells ahead of the march
+};
+template <bool CG, int W, int ROWS, int FILMS>
 __device__ __forceinline__ void heat_pair_tile(const HeatPlainArgs& a, long long t, const double* told, double* tnew,
                                                double (&acc)[2], double& rate, HeatFilmCells<ROWS, W>& xf) {
     static_assert(W == 2 || W == 4, "two or four cells of a row per thread");
+    constexpr bool AHEAD = FILMS == kFilmsAhead;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const size_t plane = (size_t)nx * ny;
     const double kf = a.kface;
@@ -629,11 +636,11 @@ __device__ __forceinline__ void heat_pair_tile(const HeatPlainArgs& a, long long
                 double shed = 0.0;
                 if (slot) shed = *slot;
                 else if (a.films.exposed && face)
-                    shed = AHEAD ? film_flux(a, i + e, j, k, c + e, t0) : film_flux_dirichlet(a, i + e, j, k, t0);
+                    shed = FILMS != kFilmsDirichlet ? film_flux(a, i + e, j, k, c + e, t0) : film_flux_dirichlet(a, i + e, j, k, t0);
                 nt[e] = t0 + a.dts * a.mobility * (flux - shed);  // add_kelvin, latent <= 0 (solid.rs:1620-1635)
                 acc[0] += a.capacity * (nt[e] - a.reference);     // solid.rs:1583-1590
                 if (shed != 0.0) acc[1] += a.dts * a.mobility * shed * a.capacity;  // solid.rs:1821-1823
-                if (AHEAD && a.radiating) {
+                if (AHEAD && !CG && a.radiating) {
                     if (slot) *slot = nt[e];
                     else if (face) rate = fmax(rate, heat_cell_rate(a, i + e, j, k, c + e, nt[e]));
                 }
@@ -648,7 +655,7 @@ __device__ __forceinline__ void heat_pair_tile(const HeatPlainArgs& a, long long
         }
         if (!ahead) break;
         __syncthreads();
-        if (a.radiating) {
+        if (!CG && a.radiating) {
             heat_film_cells(a, xf, ft, ka, kb, [&](double& slot, int fi, int fj, int fk, size_t fc) {
                 rate = fmax(rate, heat_cell_rate(a, fi, fj, fk, fc, slot));
             });
@@ -664,7 +671,7 @@ static __global__ void __launch_bounds__(256, PM_HEAT_PAIR_MIN_BLOCKS) heat_plai
     double rate = -1.0;  // a state-dependent limit: the largest rate of the new state
     __shared__ HeatFilmCells<8, 2> xf;
     for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x)
-        heat_pair_tile<false, 2, 8, AHEAD>(a, t, a.told, a.tnew, acc, rate, xf);
+        heat_pair_tile<false, 2, 8, AHEAD ? kFilmsAhead : kFilmsDirichlet>(a, t, a.told, a.tnew, acc, rate, xf);
     if (AHEAD && a.radiating) heat_rate_publish(a, rate);
     heat_plain_books(a, acc);
 }
@@ -686,7 +693,7 @@ static __global__ void __launch_bounds__(256, PM_HEAT_QUAD64_MIN_BLOCKS) heat_pl
     double rate = -1.0;  // a state-dependent limit: the largest rate of the new state
     __shared__ HeatFilmCells<8, 4> xf;
     for (long long t = blockIdx.x; t < a.tiles.ntiles; t += gridDim.x)
-        heat_pair_tile<false, 4, 8, AHEAD>(a, t, a.told, a.tnew, acc, rate, xf);
+        heat_pair_tile<false, 4, 8, AHEAD ? kFilmsAhead : kFilmsDirichlet>(a, t, a.told, a.tnew, acc, rate, xf);
     if (AHEAD && a.radiating) heat_rate_publish(a, rate);
     heat_plain_books(a, acc);
 }
@@ -786,7 +793,7 @@ __device__ __forceinline__ void heat_persist(const Args& a, const HeatPersist& p
 
 // The pair form's many-step kernel: blocks of 32 × ROWS threads (8 rows: four blocks per SM; 32 rows:
 // one block of 1024 per SM, so a 64³ block is 128 workers and the keeper).
-template <int ROWS, bool AHEAD>
+template <int ROWS, int FILMS>
 static __global__ void __launch_bounds__(32 * ROWS, ROWS == 8 ? PM_HEAT_PAIR_MIN_BLOCKS : 1)
     heat_plain_pair_steps(HeatPlainArgs a, HeatPersist p) {
     __shared__ HeatFilmCells<ROWS, 2> xf;
@@ -794,7 +801,7 @@ static __global__ void __launch_bounds__(32 * ROWS, ROWS == 8 ? PM_HEAT_PAIR_MIN
         const double* told = (s & 1) ? a.tnew : a.told;
         double* tnew = const_cast<double*>((s & 1) ? a.told : a.tnew);
         double rate = -1.0;
-        for (long long t = first; t < a.tiles.ntiles; t += stride) heat_pair_tile<true, 2, ROWS, AHEAD>(a, t, told, tnew, acc, rate, xf);
+        for (long long t = first; t < a.tiles.ntiles; t += stride) heat_pair_tile<true, 2, ROWS, FILMS>(a, t, told, tnew, acc, rate, xf);
     });
 }
 

@@ -21,9 +21,15 @@ cudaError_t launch_heat_plain_steps(const HeatPlainArgs& a, const HeatPersist& p
     HeatPersist pp = p;
     void* args[2] = {&aa, &pp};
     // the tiling's rows are the block's y extent: 8 (256 threads) or 32 (1024)
-    const bool tall = a.tiles.rows == 32, ahead = a.films.ahead != 0;
-    auto k = tall ? (ahead ? heat_plain_pair_steps<32, true> : heat_plain_pair_steps<32, false>)
-                  : (ahead ? heat_plain_pair_steps<8, true> : heat_plain_pair_steps<8, false>);
+    const bool tall = a.tiles.rows == 32;
+    // Tiles of one plane form their films in the march: forming them ahead is then two barriers a tile for
+    // one plane's films, and each film is still one thread's chain. µs a step of convective blocks, ahead
+    // and in the march: 64³ 8.79 and 7.64, 32³ 8.93 and 7.49, 16³ 7.33 and 5.75, 200 × 30 × 30 8.03 and 6.95; tiles
+    // of more planes 64 × 64 × 128 (2) 10.1 and 11.0, 96³ (4) 12.6 and 15.4, 128³ (8) 18.7 and 26.2.
+    const bool march = a.tiles.zc == 1;
+    auto k = !a.films.ahead ? (tall ? heat_plain_pair_steps<32, kFilmsDirichlet> : heat_plain_pair_steps<8, kFilmsDirichlet>)
+             : march        ? (tall ? heat_plain_pair_steps<32, kFilmsMarch> : heat_plain_pair_steps<8, kFilmsMarch>)
+                            : (tall ? heat_plain_pair_steps<32, kFilmsAhead> : heat_plain_pair_steps<8, kFilmsAhead>);
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(a.nblocks), tall ? dim3(32, 32) : tile_block(),
                                        args, 0, s);
 }
@@ -233,8 +239,8 @@ int occupancy_f64(KernelId id) {
         case kHeatPlain: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_step<true, true>, 256, 0); break;
         case kHeatPlainPair: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_step<true>, 256, 0); break;
         case kHeatPlainQuad: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_quad_step<true>, 256, 0); break;
-        case kHeatPlainSteps: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<8, true>, 256, 0); break;
-        case kHeatPlainSteps32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<32, true>, 1024, 0); break;
+        case kHeatPlainSteps: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<8, kFilmsAhead>, 256, 0); break;
+        case kHeatPlainSteps32: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, heat_plain_pair_steps<32, kFilmsAhead>, 1024, 0); break;
         case kHallF64:
             e = allow_smem(hall_step<double, false>, (int)hall_smem_bytes<double>());
             if (e != cudaSuccess) break;
