@@ -76,7 +76,8 @@ struct Hall : Handle {
         a.wsrc = wsrc;
         a.starting = starting ? 1 : 0;
         const unsigned w = wave_of(sizeof(Real) == 8 ? kHallF64 : (tma ? hall_tma_kernel_id(tshape) : kHallF32));
-        a.tiles = make_tiles(nx, ny, nz, choose_zc(nx, ny, nz, w, (sizeof(Real) == 4 && tma) ? kHallTmaShapes[tshape].planes : 2));
+        const int lo = (sizeof(Real) == 4 && tma) ? kHallTmaShapes[tshape].planes : 2;
+        a.tiles = make_tiles(nx, ny, nz, choose_hall_zc(nx, ny, nz, sm_count, w, lo));
         a.nblocks = grid_for(a.tiles, w);
         a.st = state.as<DevState>();
         a.partials = partials.as<double>();

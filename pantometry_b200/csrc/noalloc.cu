@@ -38,6 +38,7 @@ namespace {
 
 struct NoallocDevice {
     unsigned char* scratch = nullptr;  // device address of noalloc_scratch on this device
+    int sms = 0;
     int wave = 0;                      // resident blocks of the Hall kernel
 };
 
@@ -54,6 +55,7 @@ pm_status noalloc_setup(int dev, NoallocDevice& out) {
         int sms = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
+        d.sms = sms;
         d.wave = sms * blocks_per_sm(kHallF32);
         d.scratch = static_cast<unsigned char*>(ptr);
     }
@@ -108,7 +110,7 @@ extern "C" pm_status pm_hall_step_f32_noalloc(int nx, int ny, int nz, double dx,
     a.src = -1;
     a.src_i = a.src_j = a.src_k = -1;
     a.starting = 0;
-    a.tiles = make_tiles(nx, ny, nz, choose_zc(nx, ny, nz, (unsigned)d.wave, 2));
+    a.tiles = make_tiles(nx, ny, nz, choose_hall_zc(nx, ny, nz, (unsigned)d.sms, (unsigned)d.wave, 2));
     a.nblocks = grid_for(a.tiles, (unsigned)d.wave);
     // scratch layout: the state block, then 3 partial sums per block
     const size_t state_bytes = (sizeof(DevState) + 255) & ~size_t(255);

@@ -33,13 +33,32 @@ inline Tiles make_tiles(int nx, int ny, int nz, int zc, int rows = 8) {
 // does not fill the SMs takes the thinnest, since a step is then as long as one tile. Measured,
 // µs a step, chunks of 4, 8, 16 or 32 planes by their even spread alone and by this rule: a radiating f64
 // block of 150 × 121 × 93 cells 67.6 and 55.8, a filled f64 32³ one 9.9 and 6.4, a lossy f64 32 × 24 × 31
-// cavity 11.3 and 9.5, an FP32 31 × 27 × 43 one 17.2 and 15.6; a 256³ FP32 hall 96.4 and 96.4.
+// cavity 11.3 and 9.5, an FP32 31 × 27 × 43 one 17.2 and 15.6.
 inline int choose_zc(int nx, int ny, int nz, unsigned resident, int lo = 1, int off = 0) {
     int best = lo - off;
     double best_cost = -1.0;
     for (int zc = lo - off; zc < nz + lo && zc <= 64; zc += lo) {
         const long long rounds = (make_tiles(nx, ny, nz, zc).ntiles + resident - 1) / resident;
         const double cost = ((double)rounds + 0.25) * (zc + 1);
+        if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = zc; }
+    }
+    return best;
+}
+// The z-chunk of a hall's step, a multiple of its `lo` planes a stage. A hall's tile is light, so besides the
+// rounds of a block the planes count that an SM's blocks march between them, mostly on the fullest SM. Chunks
+// of more than eight stages gain nothing more. Fitted to sweeps of the chunk over 59 grids of the cp.async
+// form and 14 of the TMA one: its choices are 1.5 and 0.5 % from the best on the mean (choose_zc's 3.0 and
+// 1.6), and none is slower than chunks of 4, 8, 16 or 32 planes by their even spread by more than 4 %. Measured,
+// µs a step by choose_zc and by this: 255 × 64 × 64 nodes in FP32 16.7 and 14.8, 65 × 90 × 50 10.7 and 9.5;
+// 33 × 33 × 200 in f64 10.6 and 9.9; by TMA 64 × 64 × 256 10.6 and 10.3, 128³ 16.0 and 15.0.
+inline int choose_hall_zc(int nx, int ny, int nz, unsigned sms, unsigned resident, int lo) {
+    int best = lo;
+    double best_cost = -1.0;
+    for (int zc = lo; zc < nz + lo && zc <= 8 * lo; zc += lo) {
+        const long long tiles = make_tiles(nx, ny, nz, zc).ntiles;
+        const double mean = (double)tiles / sms, most = (double)((tiles + sms - 1) / sms);
+        const double rounds = (double)((tiles + resident - 1) / resident);
+        const double cost = (0.75 * most + 0.25 * mean + rounds) * (zc + 0.8);
         if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = zc; }
     }
     return best;

@@ -15,6 +15,10 @@ MAIN = r"""
 int main() {
     int x, y, z, wave, lo, off, near;
     while (std::scanf("%d %d %d %d %d %d %d", &x, &y, &z, &wave, &lo, &off, &near) == 7) {
+        if (near < 0) {
+            std::printf("%d 0\n", pm::choose_hall_zc(x, y, z, 148u, (unsigned)wave, lo));
+            continue;
+        }
         const unsigned w = pm::yee_tile_blocks((unsigned)wave, near != 0);
         const int zc = pm::choose_zc(x, y, z, w, lo, off);
         std::printf("%d %u\n", zc, pm::grid_for(pm::make_tiles(x, y, z, zc), w));
@@ -59,3 +63,17 @@ def test_a_cavitys_chunk_is_the_best_for_the_blocks_that_take_its_tiles(rules, w
         assert grid == min(blocks, _tiles(x, y, z, zc))
         chunks = range(lo - 1, min(65, z + lo), lo)
         assert zc in chunks and cost(zc) == min(cost(c) for c in chunks), (x, y, z, zc)
+
+
+@pytest.mark.parametrize("wave,lo", [(444, 2), (296, 2), (296, 8)])
+def test_a_halls_chunk_is_the_best_by_its_rounds_and_its_sms_planes(rules, wave, lo):
+    r = random.Random(6)
+    sizes = [(255, 64, 64), (128, 128, 128), (33, 33, 200), (3, 3, 3), (2, 2, 2)]
+    sizes += [tuple(r.randint(2, 260) for _ in range(3)) for _ in range(400)]
+    for (x, y, z), (zc, _) in zip(sizes, rules([(*s, wave, lo, 0, -1) for s in sizes])):
+        def cost(c):
+            t = _tiles(x, y, z, c)
+            return (0.75 * -(-t // 148) + 0.25 * (t / 148) + -(-t // wave)) * (c + 0.8)
+
+        chunks = range(lo, min(8 * lo + 1, z + lo), lo)
+        assert zc in chunks and cost(zc) <= min(cost(c) for c in chunks) * (1 + 1e-12), (x, y, z, zc)
