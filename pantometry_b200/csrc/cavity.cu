@@ -845,33 +845,17 @@ pm_status pm_cavity_create(const pm_cavity_desc* d, pm_cavity** out) {
     c->uniform_media();
     pm_status s = c->init(d->device, 0);
     if (s != PM_OK) { delete c; return s; }
-    // Padded rows start on 32-byte sectors: with TMA's own 16 bytes every store of a warp's 32 nodes
-    // cut a sector in two at both ends on every other row (384³ 560 -> 528 us a step, 256³ 174 -> 160,
-    // 160³ 51.4 -> 48.9, 128³ of mixed ε 37.5 -> 36.8; 96³, which L2 holds, 17.2 both ways). Whole 128-byte lines gave 384³ 517 but 96³ 17.6 and 128³ of mixed ε 38.3: the
-    // wider rows crowd a lattice out of L2. Four floats stay for a lattice only they leave indexable
-    // by 32 bits, or that the memory left holds.
-    const unsigned narrow = (unsigned)((c->nx + 1 + 3) & ~3);
-    c->L = (unsigned)((c->nx + 1 + 7) & ~7);
-    if (c->lattice() >= (1ull << 32)) c->L = narrow;
+    size_t free_bytes = 0, total_bytes = 0;
+    if (c->precision != PM_FIELDS_F32 || cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) free_bytes = 0;
+    c->L = cavity_row_pitch(c->nx, c->ny, c->nz, free_bytes);
     c->tma = c->precision == PM_FIELDS_F32 && c->lattice() < (1ull << 32);
-    auto alloc_fields = [&]() -> cudaError_t {
+    for (int attempt = 0; attempt < 2; ++attempt) {
         for (int par = 0; par < 2; ++par)
             for (int q = 0; q < 6; ++q) {
-                if (cudaError_t e = c->f[par][q].alloc(c->dcount(q) * c->esize()); e != cudaSuccess) return e;
+                cudaError_t e = c->f[par][q].alloc(c->dcount(q) * c->esize());
+                if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaMalloc cavity fields"); }
                 cudaMemset(c->f[par][q].p, 0, c->dcount(q) * c->esize());
             }
-        return cudaSuccess;
-    };
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        cudaError_t e = alloc_fields();
-        if (e == cudaErrorMemoryAllocation && c->tma && c->L != narrow) {
-            (void)cudaGetLastError();
-            for (auto& par : c->f)
-                for (auto& q : par) q.release();
-            c->L = narrow;
-            e = alloc_fields();
-        }
-        if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaMalloc cavity fields"); }
         // a shape the driver will not tile steps with the cp.async kernel on the reference layout
         if (!c->tma || c->build_maps() == PM_OK) break;
         c->tma = false;

@@ -2,6 +2,8 @@
 // plain C++ compiler takes too.
 #pragma once
 
+#include <stddef.h>
+
 namespace pm {
 
 // The tiling every step kernel walks: 32 × 8 columns of cells (one warp row per y), each
@@ -70,6 +72,18 @@ inline int choose_hall_zc(int nx, int ny, int nz, unsigned sms, unsigned residen
 // whose last round is a few tiles long, lose as they leave their thin chunks: 59 × 46 × 146 13.5 and 14.4,
 // 64 × 32 × 256 of mixed ε 17.1 and 18.2.
 inline unsigned yee_tile_blocks(unsigned wave, bool near) { return near && wave > 1 ? wave - 1 : wave; }
+// The row pitch, in floats, of a cavity's padded FP32 lattice. Rows start on 32-byte sectors: with the 16
+// bytes that TMA asks for, every store of a warp's 32 nodes cut a sector in two at both ends on every other
+// row (384³ 560 -> 528 us a step, 256³ 174 -> 160, 160³ 51.4 -> 48.9, 128³ of mixed ε 37.5 -> 36.8; 96³, which
+// L2 holds, 17.2 both ways). Whole 128-byte lines gave 384³ 517 but 96³ 17.6 and 128³ of mixed ε 38.3: the
+// wider rows crowd a lattice out of L2. Four floats stay for a lattice that only they leave indexable by 32
+// bits, and where the free memory may not hold all that a cavity ever allocates at the wider pitch: two sets
+// of fields, three gains, Mur's three, a checkpoint's six, and media, masks and staging of 24 arrays' size.
+inline unsigned cavity_row_pitch(int nx, int ny, int nz, size_t free_bytes) {
+    const unsigned narrow = (unsigned)((nx + 1 + 3) & ~3), wide = (unsigned)((nx + 1 + 7) & ~7);
+    const size_t lattice = (size_t)wide * ((size_t)ny + 1) * ((size_t)nz + 1);
+    return lattice < ((size_t)1 << 32) && lattice <= free_bytes / (48 * sizeof(float)) ? wide : narrow;
+}
 inline unsigned grid_for(const Tiles& t, unsigned resident) {
     return (unsigned)(t.ntiles < (long long)resident ? t.ntiles : (long long)resident);
 }

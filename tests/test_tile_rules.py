@@ -15,6 +15,10 @@ MAIN = r"""
 int main() {
     int x, y, z, wave, lo, off, near;
     while (std::scanf("%d %d %d %d %d %d %d", &x, &y, &z, &wave, &lo, &off, &near) == 7) {
+        if (near == -2) {  // the wave in MiB of free memory
+            std::printf("%u 0\n", pm::cavity_row_pitch(x, y, z, (size_t)wave << 20));
+            continue;
+        }
         if (near < 0) {
             std::printf("%d 0\n", pm::choose_hall_zc(x, y, z, 148u, (unsigned)wave, lo));
             continue;
@@ -77,3 +81,16 @@ def test_a_halls_chunk_is_the_best_by_its_rounds_and_its_sms_planes(rules, wave,
 
         chunks = range(lo, min(8 * lo + 1, z + lo), lo)
         assert zc in chunks and cost(zc) <= min(cost(c) for c in chunks) * (1 + 1e-12), (x, y, z, zc)
+
+
+def test_a_cavitys_rows_widen_only_where_all_it_may_allocate_fits(rules):
+    r = random.Random(7)
+    sizes = [(384, 384, 384), (383, 383, 383), (2047, 1447, 1446), (1619, 1625, 1625), (1, 1, 1), (1275, 1275, 1275)]
+    sizes += [tuple(r.randint(1, 1400) for _ in range(3)) for _ in range(200)]
+    for free in (0, 16, 1 << 14, 170 << 10):  # MiB
+        for (x, y, z), (pitch, _) in zip(sizes, rules([(*s, free, 0, 0, -2) for s in sizes])):
+            wide, narrow = (x + 8) // 8 * 8, (x + 4) // 4 * 4
+            lattice = wide * (y + 1) * (z + 1)
+            fits = lattice < 1 << 32 and 48 * 4 * lattice <= free << 20
+            assert pitch == (wide if fits else narrow), (x, y, z, free)
+            assert pitch >= x + 1
