@@ -673,21 +673,28 @@ struct Cavity : Handle {
     }
 
     // The padded cavity back to the reference layout (before media with conductivity or per-cell
-    // μ, which only the cp.async kernel reads). The state goes through the host once; a
-    // checkpoint taken in the other layout is dropped.
+    // μ, which only the cp.async kernel reads). The state and a kept history go through the host once;
+    // a checkpoint taken in the other layout is dropped.
     pm_status leave_tma() {
         if (!tma) return PM_OK;
-        std::vector<double> v[6];
+        std::vector<double> v[9];
         pm_status s;
-        for (int q = 0; q < 6; ++q) {
-            v[q].resize(count(q));
-            if ((s = get(q, v[q].data())) != PM_OK) return s;
+        for (int q = 0; q < (use_stale ? 9 : 6); ++q) {
+            v[q].resize(count(q % 6));
+            if (q >= 6) std::swap(f[parity][q - 6].p, stale[q - 6].p);
+            s = get(q % 6, v[q].data());
+            if (q >= 6) std::swap(f[parity][q - 6].p, stale[q - 6].p);
+            if (s != PM_OK) return s;
         }
         tma = false;
         drop_graphs();
         has_saved = false;
-        for (int q = 0; q < 6; ++q)
-            if ((s = put(q, v[q].data())) != PM_OK) return s;
+        for (int q = 0; q < (use_stale ? 9 : 6); ++q) {
+            if (q >= 6) std::swap(f[parity][q - 6].p, stale[q - 6].p);
+            s = put(q % 6, v[q].data());
+            if (q >= 6) std::swap(f[parity][q - 6].p, stale[q - 6].p);
+            if (s != PM_OK) return s;
+        }
         PM_CUDA(cudaStreamSynchronize(stream()));
         return PM_OK;
     }
