@@ -395,13 +395,14 @@ struct Cavity : Handle {
     // box. A conducting wall counts too: it may be set open after these steps, and its first update then
     // reads the history that they left.
     int solid_lo[3] = {0, 0, 0}, solid_hi[3] = {0, 0, 0};  // the solid cells' least and greatest indices
-    bool solid_after_walls() const {
-        if (!any_solid || !open_or_magnetic()) return false;
+    bool solid_near_wall() const {
+        if (!any_solid) return false;
         const int n[3] = {nx, ny, nz};
         for (int a = 0; a < 3; ++a)
             if (solid_lo[a] <= 1 || solid_hi[a] >= n[a] - 2) return true;
         return false;
     }
+    bool solid_after_walls() const { return open_or_magnetic() && solid_near_wall(); }
     pm_status ensure_stale() {
         for (int q = 0; q < 3; ++q) {
             const size_t bytes = dcount(q) * esize();
@@ -409,17 +410,36 @@ struct Cavity : Handle {
         }
         return PM_OK;
     }
-    // Before E is rewritten between steps: keep the history the next step's open walls need.
-    pm_status keep_history() {
-        if (!has_prev || use_stale) return PM_OK;
-        for (int q = 0; q < 3; ++q) {
-            const size_t bytes = dcount(q) * esize();
-            if (stale[q].bytes < bytes) PM_CUDA(stale[q].alloc(bytes));
-            PM_CUDA(cudaMemcpyAsync(stale[q].p, f[parity][q].p, bytes, cudaMemcpyDeviceToDevice, stream()));
+    // The history the last step left, into `stale`: its E, and where conducting walls let the step zero the
+    // edges of an obstacle beside one (zeroed_dt: that step's size), what they held before.
+    double zeroed_dt = NAN;
+    pm_status history_to_stale() {
+        pm_status s = ensure_stale();
+        if (s != PM_OK) return s;
+        for (int q = 0; q < 3; ++q)
+            PM_CUDA(cudaMemcpyAsync(stale[q].p, f[parity][q].p, dcount(q) * esize(), cudaMemcpyDeviceToDevice, stream()));
+        if (!std::isnan(zeroed_dt)) {
+            if ((s = prepare_coefs(zeroed_dt)) != PM_OK) return s;
+            PM_CUDA(precision == PM_PLAIN_F64 ? obstacle_history<double>() : obstacle_history<float>());
         }
         use_stale = true;
         return PM_OK;
     }
+    template <typename Real>
+    cudaError_t obstacle_history() const {
+        YeeHistoryArgs<Real> a{};
+        a.s = sargs<Real>(parity ^ 1, zeroed_dt);
+        for (int q = 0; q < 6; ++q) {
+            if (q < 3) a.hist[q] = stale[q].as<Real>();
+            int ex, ey, ez;
+            extents(q, ex, ey, ez);
+            a.rx[q] = tma ? L : (unsigned)ex;
+            a.ry[q] = tma ? (unsigned)(ny + 1) : (unsigned)ey;
+        }
+        return launch_yee_obstacle_history<Real>(a, stream());
+    }
+    // Before E is rewritten between steps: keep the history the next step's open walls need.
+    pm_status keep_history() { return !has_prev || use_stale ? PM_OK : history_to_stale(); }
     // The walls after the step from `par` into `par ^ 1` (cavity.rs:1074-1164): magnetic mirrors,
     // then open walls by Mur (or held at zero before any history exists).
     template <typename Real>
@@ -887,6 +907,8 @@ pm_status pm_cavity_fill_cells(pm_cavity* cp, const double* eps_r, const double*
         if (mu_r) c->cell_mu[q] = mu_r[q];
         if (sigma) c->cell_sig[q] = sigma[q];
     }
+    if (!std::isnan(c->zeroed_dt))
+        if (pm_status ks = c->keep_history(); ks != PM_OK) return ks;  // while the last step's media are at hand
     c->uniform = false;
     c->refresh_media();
     // the TMA-staged kernel steps per-cell ε with no conductivity and one μ on the padded layout;
@@ -1076,14 +1098,7 @@ pm_status pm_cavity_step(pm_cavity* cp, double dt, long long nsteps, pm_violatio
     if (c->solid_after_walls()) {
         pm_status es = c->ensure_stale();
         if (es != PM_OK) return es;
-        if (c->has_prev && !c->use_stale) {
-            // the history the last step left, now kept in `stale` (stepped before these walls were
-            // set: the field after its step, the obstacles' edges already zeroed)
-            for (int q = 0; q < 3; ++q)
-                PM_CUDA(cudaMemcpyAsync(c->stale[q].p, c->f[c->parity][q].p, c->dcount(q) * c->esize(), cudaMemcpyDeviceToDevice,
-                                        c->stream()));
-            c->use_stale = true;
-        }
+        if ((es = c->keep_history()) != PM_OK) return es;  // kept in `stale` from here on
     }
     // cavity.rs:1469-1480
     const double h = dt, limit = c->courant_limit();
@@ -1114,6 +1129,7 @@ pm_status pm_cavity_step(pm_cavity* cp, double dt, long long nsteps, pm_violatio
     }
     s = c->run_steps(remaining, dt, true, [c, h](int par, cudaStream_t st) { return c->step_once(par, h, true, false, st); });
     if (s != PM_OK) return s;
+    c->zeroed_dt = c->solid_near_wall() && !c->open_or_magnetic() ? h : NAN;
     return c->finish_call(before, out, "simulation", "simulation", true);
 }
 

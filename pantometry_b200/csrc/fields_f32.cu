@@ -218,6 +218,11 @@ cudaError_t launch_yee_enforce_solid<float>(const YeeWallArgs<float>& a, const u
     return cudaGetLastError();
 }
 template <>
+cudaError_t launch_yee_obstacle_history<float>(const YeeHistoryArgs<float>& a, cudaStream_t s) {
+    yee_obstacle_history<float><<<kMeasureBlocks, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+template <>
 cudaError_t launch_yee_walls<float>(const YeeWallArgs<float>& a, cudaStream_t s) {
     yee_walls<float><<<std::min((a.first[6] + 255u) / 256u, (unsigned)kMeasureBlocks), 256, 0, s>>>(a);
     return cudaGetLastError();

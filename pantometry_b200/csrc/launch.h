@@ -97,6 +97,7 @@ template <typename Real> cudaError_t launch_yee_measure(const YeeHArgs<Real>& a,
 template <typename Real> cudaError_t launch_yee_walls(const YeeWallArgs<Real>& a, cudaStream_t s);
 template <typename Real>
 cudaError_t launch_yee_enforce_solid(const YeeWallArgs<Real>& a, const uint8_t* solid, cudaStream_t s);
+template <typename Real> cudaError_t launch_yee_obstacle_history(const YeeHistoryArgs<Real>& a, cudaStream_t s);
 template <typename Real> cudaError_t launch_yee_coefs(const YeeCoefArgs<Real>& a, cudaStream_t s);
 // The FP32 Hall step staged by TMA (padded face layout, nx a multiple of 4), in tile shape `shape`
 // (an index of kHallTmaShapes).

@@ -101,6 +101,11 @@ cudaError_t launch_yee_enforce_solid<double>(const YeeWallArgs<double>& a, const
     return cudaGetLastError();
 }
 template <>
+cudaError_t launch_yee_obstacle_history<double>(const YeeHistoryArgs<double>& a, cudaStream_t s) {
+    yee_obstacle_history<double><<<kMeasureBlocks, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+template <>
 cudaError_t launch_yee_walls<double>(const YeeWallArgs<double>& a, cudaStream_t s) {
     yee_walls<double><<<std::min((a.first[6] + 255u) / 256u, (unsigned)kMeasureBlocks), 256, 0, s>>>(a);
     return cudaGetLastError();

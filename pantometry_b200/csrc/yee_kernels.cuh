@@ -696,6 +696,52 @@ static __global__ void yee_enforce_solid(YeeWallArgs<Real> a, const uint8_t* __r
     }
 }
 
+// What the obstacles' edges held after the last step's update and before they were zeroed (cavity.rs:
+// 1383-1452, from that step's old E and its new H), into Mur's history: after steps between conducting walls
+// only, where the step kernels zero those edges and no history is kept beside E. `s` holds the last step's
+// arguments; component c's value (i, j, k) is at i + rx[c]·(j + ry[c]·k).
+template <typename Real>
+struct YeeHistoryArgs {
+    YeeStepArgs<Real> s;
+    Real* hist[3];
+    unsigned rx[6], ry[6];
+};
+template <typename Real>
+static __global__ void yee_obstacle_history(const __grid_constant__ YeeHistoryArgs<Real> a) {
+    const YeeStepArgs<Real>& s = a.s;
+    const int nx = s.nx, ny = s.ny, nz = s.nz;
+    const size_t nodes = (size_t)(nx + 1) * (ny + 1) * (nz + 1);
+    const long long last = s.st->steps - 1;
+    const double jsrc = (s.src_i >= 0 && last >= 0 && last < s.ncurrent) ? s.current[last] : 0.0;
+    for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < nodes; r += (size_t)gridDim.x * blockDim.x) {
+        const unsigned bits = s.solid[r];
+        if (!bits) continue;
+        const int i = (int)(r % (size_t)(nx + 1)), j = (int)(r / (size_t)(nx + 1) % (size_t)(ny + 1)),
+                  k = (int)(r / ((size_t)(nx + 1) * (ny + 1)));
+        auto at = [&](int c, int ii, int jj, int kk) { return (size_t)ii + (size_t)a.rx[c] * ((size_t)jj + (size_t)a.ry[c] * (size_t)kk); };
+        auto h = [&](int c, int ii, int jj, int kk) { return s.neu[c][at(c, ii, jj, kk)]; };
+        const bool ix = i >= 1 && i < nx, iy = j >= 1 && j < ny, iz = k >= 1 && k < nz;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const bool interior = q == 0 ? (iy && iz) : q == 1 ? (ix && iz) : (ix && iy);
+            if (!((bits >> q) & 1) || !interior) continue;
+            Real curl;
+            if (q == 0) curl = (h(5, i, j, k) - h(5, i, j - 1, k)) - (h(4, i, j, k) - h(4, i, j, k - 1));
+            else if (q == 1) curl = (h(3, i, j, k) - h(3, i, j, k - 1)) - (h(5, i, j, k) - h(5, i - 1, j, k));
+            else curl = (h(4, i, j, k) - h(4, i - 1, j, k)) - (h(3, i, j, k) - h(3, i, j - 1, k));
+            const size_t n = at(q, i, j, k);
+            const Real gain = s.uniform ? s.gain[q] : s.cgain[q][n];
+            const Real decay = (s.uniform || s.lossless) ? s.decay[q] : s.cdecay[q][n];
+            Real v = decay * s.old[q][n] + gain * curl;
+            if (q == 2 && i == s.src_i && j == s.src_j && k == s.src_k) {
+                const double e = s.eps_src, ss = s.sig_src;
+                v = (Real)((double)v - (s.dt / e) / (1.0 + (ss * s.dt / (2.0 * e))) * jsrc);
+            }
+            a.hist[q][n] = v;
+        }
+    }
+}
+
 // A wall's rank in the reference's order, −1 for a wall that is not this launch's.
 template <typename Real>
 __device__ __forceinline__ int yee_wall_rank(const YeeWallArgs<Real>& a, int w) {
