@@ -143,7 +143,8 @@ __device__ __forceinline__ void yee_tma_close(DevState* st, const double (&acc)[
 constexpr int kNearWidth = 5;  // lattice nodes of the box along each axis
 struct YeeNearArgs {
     const float* old[6];    // ex ey ez hx hy hz at step n, padded lattice
-    float* neu[6];          // at n + 1, already stepped by yee_tma_step
+    float* neu[6];          // at n + 1: written here while the tiles run, never read; the box's faces and edges and the
+                            // ring's edges, exactly the nodes near_left takes from the tiles
     const double* nold;     // the box's f64 values at step n: [q][lk][lj][li], w³ per component
     double* nneu;           // at n + 1
     int x0, y0, z0, w;      // the box: w³ lattice nodes from (x0, y0, z0)
