@@ -3,6 +3,7 @@
 #include <cudaTypedefs.h>
 
 #include "launch.h"
+#include "room_launch.cuh"
 
 namespace pm {
 
@@ -238,50 +239,8 @@ cudaError_t launch_room<float>(const RoomArgs<float>& a, cudaStream_t s) {
     room_step<float><<<a.nblocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
-// One cluster of room_steps: its launch, and the largest one that holds a room.
-template <typename Real>
-static cudaError_t room_steps_config(cudaLaunchConfig_t& c, cudaLaunchAttribute& at, int blocks, size_t smem, cudaStream_t s) {
-    if (cudaError_t e = allow_smem(room_steps<Real>, (int)smem); e != cudaSuccess) return e;
-    if (blocks > 8)
-        if (cudaError_t e = cudaFuncSetAttribute(room_steps<Real>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            e != cudaSuccess)
-            return e;
-    c = cudaLaunchConfig_t{};
-    c.gridDim = dim3((unsigned)blocks);
-    c.blockDim = dim3(kRoomThreads + 32);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaSuccess;
-}
-template <>
-cudaError_t launch_room_steps<float>(const RoomStepsArgs<float>& a, int blocks, cudaStream_t s) {
-    cudaLaunchConfig_t c;
-    cudaLaunchAttribute at;
-    if (cudaError_t e = room_steps_config<float>(c, at, blocks, room_steps_smem<float>(a.nx, a.rows), s); e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&c, room_steps<float>, a);
-}
-template <>
-int room_steps_cluster<float>(int nx, int ny, int* rows) {
-    for (int blocks = kRoomMaxCluster; blocks >= 1; blocks /= 2) {
-        if (blocks > ny) continue;
-        *rows = (ny + blocks - 1) / blocks;
-        const size_t smem = room_steps_smem<float>(nx, *rows);
-        if (smem > 200 * 1024) break;  // a smaller cluster's blocks hold more rows
-        cudaLaunchConfig_t c;
-        cudaLaunchAttribute at;
-        int fit = 0;
-        if (room_steps_config<float>(c, at, blocks, smem, nullptr) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&fit, room_steps<float>, &c) == cudaSuccess && fit > 0)
-            return blocks;
-        cudaGetLastError();  // a cluster the device does not take is not an error of the stream
-    }
-    return 0;
-}
+template cudaError_t launch_room_steps<float>(const RoomStepsArgs<float>&, int, cudaStream_t);
+template int room_steps_cluster<float>(int, int, int*);
 template <>
 cudaError_t launch_room_measure<float>(const RoomMeasureArgs<float>& a, cudaStream_t s) {
     room_measure<float><<<a.nblocks, 256, 0, s>>>(a);
