@@ -680,7 +680,8 @@ static __global__ void __launch_bounds__(256, PM_HEAT_PAIR_MIN_BLOCKS) heat_plai
 // thread, where the reference's sequential flux sum makes each cell one chain. The latency of each
 // plane's loads bounds it, so the warps in flight: a Dirichlet 256³ block ran 188 Gcell/s at two blocks
 // of 256 per SM (96 registers), 203 at three (80) and 180 at four (64, spilled); a convective
-// 256 × 240 × 224 one, whose films are formed ahead, 123, 132 and 104. Tried beside it: each face's product
+// 256 × 240 × 224 one, whose films are formed ahead, 123, 132 and 104; a small radiating block, bound by its
+// films' own latency, loses a little (52 × 41 × 41: 21.3 us a step at two blocks, 22.4 at three). Tried beside it: each face's product
 // formed once for its two cells (a fifth fewer FP64 instructions, 1 % either way), the next plane's rows
 // loaded a plane ahead (209 at two blocks for Dirichlet, 123 for films).
 #ifndef PM_HEAT_QUAD64_MIN_BLOCKS

@@ -37,10 +37,10 @@ struct YeeMaps {
 };
 
 // The tile shapes of each form: planes per stage, stages in the ring, resident blocks per SM the
-// kernel is held to. Shape 0 of each is the one hand sweeps chose on B200 at 384³: one medium 3
-// planes × 2 stages at three blocks per SM (61 KB of shared memory a block, 384³ in 512 us a step
-// against 668 for 4 × 2 and 644 for 3 × 3 at two), mixed ε 4 × 2 at two (95 KB with its gain boxes,
-// 85 Gcell/s against 60 for 3 × 2 at three). The others are the runners-up, which pm_cavity_autotune times on a cavity's own grid.
+// kernel is held to. Shape 0 of each is the fastest on B200 at 384³, calls of 64 steps at 1965 MHz: one
+// medium 3 planes × 2 stages at three blocks per SM (61 KB of shared memory a block; 503 us a step without
+// a source, 537 for 4 × 2 and 528 for 3 × 3 at two), mixed ε 4 × 2 at two (102 KB with its gain boxes; 622 us
+// a step, 655 for 3 × 2). The others are the runners-up, which pm_cavity_autotune times on a cavity's own grid.
 // Every shape computes each edge and face with the same expressions, so they agree bit for bit.
 struct YeeTmaShape {
     int planes, stages, min_blocks;
